@@ -29,7 +29,7 @@ NVCC_FLAGS = [
 
 
 # the sources every decoder of the runtime needs, and each decoder's own
-RUNTIME = ("core", "tensor_map", "gemm_tc", "model_loader", "runtime")
+RUNTIME = ("core", "tensor_map", "gemm_tc", "model_loader", "runtime", "skinny_tc")
 DECODERS = {"Llama": ("decoder_gqa", "decode", "prefill"), "Maposun": ("decoder_latent", "latent_attn", "latent_prefill"),
             "Vofusun": ("decoder_hybrid", "grouped_attn", "grouped_prefill", "delta_rule")}
 

@@ -29,7 +29,8 @@ enum Knob {
     KNOB_RUNTIME_PDL,           // 1: skinny kernels launch as programmatic dependents (weights prefetched before the wait)
     KNOB_RUNTIME_ROPE_FUSED,    // 1: RoPE + KV scatter in the Q/K/V projection's epilogue, 0: separate kernel
     KNOB_RUNTIME_SKINNY,        // decode-step projections: 0 library GEMMs, 1 skinny_gemm_kernel (W in registers),
-                                // 2 skinny_stream_kernel (W through shared memory; default)
+                                // 2 chosen from the shape (default): skinny_stream_kernel (W through shared memory) or
+                                // skinny_tc_kernel (K split over a cluster, tcgen05), 3 skinny_tc_kernel
     KNOB_SCAN16_LANE,           // 1: 16-bit scans hold a whole segment per lane, 0: four lanes per segment
     KNOB_RUNTIME_GEMM,          // prefill projections: 1 the tcgen05 GEMM of this library (default), 0 library GEMMs
     KNOB_GEMM_TILE_N,           // 128 or 256: force the tensor-core GEMM's tile width (0: chosen from the shape)
@@ -40,6 +41,7 @@ enum Knob {
     KNOB_DELTA_PLAIN,           // 1: the gated delta rule token by token on the plain kernel
     KNOB_DELTA_COLUMNS,         // 1, 2 or 4: columns of S per lane (tensor-core form: 4, 2 or 1 warps per 16 columns) in the walk over blocks
     KNOB_DELTA_TENSOR,          // 0: blocks of 16-bit sessions without tensor cores as well
+    KNOB_SKINNY_CLUSTER,        // 1..8: CTAs that share K in skinny_tc_kernel (0: chosen from the shape)
     KNOB_COUNT
 };
 

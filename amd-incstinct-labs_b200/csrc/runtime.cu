@@ -541,6 +541,8 @@ extern "C" int b200p_skinny_gemm(int dtype, int prologue, int epilogue, const vo
     if (sm_count() <= 0) return B200P_E_NO_DEVICE;
     SkinnyArgs a{};
     a.W = W; a.X16 = x16; a.X32 = x32; a.norm_w = norm_w; a.out = out; a.M = M; a.N = N; a.K = K; a.ldx = ldx; a.ldo = ldo; a.eps = eps;
+    // the entry's own limit (rows of X in one CTA's shared memory); the runtime's longer rows take the split kernel
+    if (tuning(KNOB_RUNTIME_SKINNY, 2) != 3 && !skinny_rows_fit(M, K)) return B200P_E_RANGE;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto run = [&](auto tag) -> int {
         using T = decltype(tag);

@@ -787,30 +787,18 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
     }
 }
 
-// Launch: returns B200P_E_RANGE when the shape is outside the kernel's domain (the caller then
-// takes the library GEMM).  K must be a multiple of 16 (32-byte steps along the rows of W and X),
-// ldx of 8, W 32-byte aligned.
-template <typename T, int PRO, int EPI, int MH>
-int launch_skinny_mh(const SkinnyArgs& a, cudaStream_t st);
-
-// Up to 8 rows of X: one B fragment per A fragment; 9 .. 16 rows: two.
-template <typename T, int PRO, int EPI>
-int launch_skinny(const SkinnyArgs& a, cudaStream_t st) {
-    return a.M <= 8 ? launch_skinny_mh<T, PRO, EPI, 1>(a, st) : launch_skinny_mh<T, PRO, EPI, 2>(a, st);
+// Whether M rows of K columns of X fit the shared memory of these kernels.
+inline bool skinny_rows_fit(int M, int K) {
+    return M <= kSkinnyMaxM && size_t(M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16) * size_t(K + kSkinnyXPad) * 2 <= 190 * 1024;
 }
 
+// Launch of shapes in skinny_domain (skinny_tc.cuh, which chooses between these kernels and its own); B200P_E_RANGE: they
+// do not fit these kernels either.
 template <typename T, int PRO, int EPI, int MH>
 int launch_skinny_mh(const SkinnyArgs& a, cudaStream_t st) {
-    if (a.M < 1 || a.M > kSkinnyMaxM || a.K < 16 || a.K % 16 != 0 || a.N < 1) return B200P_E_RANGE;
-    if (PRO == PRO_PLAIN && (a.ldx % 8 != 0 || !aligned(a.X16, 16))) return B200P_E_RANGE;
-    if (PRO == PRO_RMSNORM && (!aligned(a.X32, 16) || !aligned(a.norm_w, 8) || a.ldx32 % 4 != 0)) return B200P_E_RANGE;
-    if (PRO == PRO_POSTADD && (!aligned(a.X32, 16) || !aligned(a.Y32, 16) || !aligned(a.x_out, 16) || !aligned(a.norm_w, 8))) return B200P_E_RANGE;
-    if (EPI == EPI_PAIRROT && (a.pair.plain % 16 != 0 || a.pair.rotated % 16 != 0 || a.N != a.pair.heads * (a.pair.plain + a.pair.rotated))) return B200P_E_RANGE;
-    if (!aligned(a.W, 16)) return B200P_E_RANGE;               // bulk copies need 16 bytes; the register kernel's 32-byte loads are checked below
+    if (!skinny_rows_fit(a.M, a.K)) return B200P_E_RANGE;
     const int Mp = a.M <= 1 ? 1 : a.M <= 2 ? 2 : a.M <= 4 ? 4 : a.M <= 8 ? 8 : 16;
     const size_t smem = size_t(Mp) * (a.K + kSkinnyXPad) * 2;
-    if (smem > 190 * 1024) return B200P_E_RANGE;
-    if (EPI == EPI_ROPE && (a.rope.D % 16 != 0 || a.N != (a.rope.nQH + 2 * a.rope.nKVH) * a.rope.D)) return B200P_E_RANGE;
     const int sms = sm_count() > 0 ? sm_count() : 148;
     constexpr bool paired = epi_paired(EPI);
     const bool pdl = tuning(KNOB_RUNTIME_PDL, 1) != 0;

@@ -63,6 +63,16 @@ __host__ __device__ constexpr uint32_t instr_desc_f16(int M, int N, int fmt, int
          | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
 }
 
+// One thread of a converged warp.  The issuing warp runs its loop with all 32 lanes and takes this branch only around the
+// MMAs and commits: descriptors, addresses and barriers then stay in uniform registers.  Behind `if (lane == 0)` every
+// operand is moved there one by one (measured, M = 128, N = 16: four MMAs, commit, wait for a completed barrier 484 cycles,
+// in this form 357; four MMAs alone 188 and 161).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 // ---- MMA (issued by ONE thread) ------------------------------------------------------------
 // D[tmem] (+)= A[smem] * B[smem];  accumulate = 0 overwrites D.
 __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
@@ -86,6 +96,14 @@ __device__ __forceinline__ void commit(uint64_t* bar) {
 __device__ __forceinline__ void ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr) : "memory");
+}
+template <int N> __device__ __forceinline__ void ld_32x32b(uint32_t taddr, uint32_t* r) {
+    static_assert(N == 4 || N == 8, "narrow loads");
+    if constexpr (N == 4)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+    else
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"

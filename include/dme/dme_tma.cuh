@@ -54,6 +54,26 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
+// Asks without waiting (try_wait may suspend the thread for a while when the phase is still running).
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+// try_wait with cluster scope: what other CTAs of the cluster wrote before (or with) the phase's completion is visible.
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
 __device__ __forceinline__ uint64_t global_timer_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -64,13 +84,15 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
 // `abort_flag` (optional, global memory): a word that is non-zero once ANY wait of the launch has
 // given up; every other wait then gives up at its next check instead of running out its own limit, so
 // a launch whose pipeline is broken ends within about one limit, not one limit per CTA.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, int* abort_flag = nullptr) {
-    if (mbar_try_wait(bar, parity)) return true;
+    auto done = [&] { return CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
+    if (done()) return true;
     const uint64_t t0 = global_timer_ns();
     for (;;) {
         #pragma unroll 1
         for (int i = 0; i < 256; ++i)
-            if (mbar_try_wait(bar, parity)) return true;
+            if (done()) return true;
         if (abort_flag && *reinterpret_cast<volatile int*>(abort_flag) != 0) return false;
         if (global_timer_ns() - t0 > kWaitLimitNs) {
             if (abort_flag) atomicExch(abort_flag, 1);
@@ -109,6 +131,10 @@ __device__ __forceinline__ void prefetch_l2(const void* gmem_src, uint32_t bytes
 __device__ __forceinline__ void copy_tile_2d(void* smem_dst, const void* tensor_map, int x, int y, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  :: "r"(smem_addr(smem_dst)), "l"(tensor_map), "r"(smem_addr(bar)), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void copy_tile_2d_stream(void* smem_dst, const void* tensor_map, int x, int y, uint64_t* bar, uint64_t policy) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+                 :: "r"(smem_addr(smem_dst)), "l"(tensor_map), "r"(smem_addr(bar)), "r"(x), "r"(y), "l"(policy) : "memory");
 }
 __device__ __forceinline__ void copy_tile_4d(void* smem_dst, const void* tensor_map, int x, int y, int z, int w, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"

@@ -138,29 +138,31 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap mapA, con
         }
     } else if (warp == 1) {
         // ---------------------------------- MMA issuer ------------------------------------
-        if (lane == 0) {
-            constexpr uint32_t idesc = tc::instr_desc_f16(kTM, BN, GFmt<T>::id, 0, 0);
-            dme::Ring<ST> r;
-            int it = 0;
-            for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++it) {
-                const int b = it & 1;
-                // the epilogue of the tile that used this accumulator buffer two tiles ago must have read it
-                if (it >= 2 && !dme::wait(&acc_empty[b], uint32_t(((it >> 1) - 1) & 1), p.abort_word)) { ok = false; break; }
+        // all lanes walk the loop and wait; one issues (tc::elect_one)
+        constexpr uint32_t idesc = tc::instr_desc_f16(kTM, BN, GFmt<T>::id, 0, 0);
+        auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, dme::wait(bar, parity, p.abort_word)) != 0; };
+        const uint64_t a0 = tc::smem_desc_sw128(dme::smem_addr(smem), 16, 1024);
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        dme::Ring<ST> r;
+        int it = 0;
+        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++it) {
+            const int b = it & 1;
+            // the epilogue of the tile that used this accumulator buffer two tiles ago must have read it
+            if (it >= 2 && !wait(&acc_empty[b], uint32_t(((it >> 1) - 1) & 1))) { ok = false; break; }
+            tc::fence_after_sync();
+            for (int kb = 0; kb < kblocks; ++kb) {
+                if (!wait(&full[r.stage], r.phase)) { ok = false; break; }
                 tc::fence_after_sync();
-                for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!dme::wait(&full[r.stage], r.phase, p.abort_word)) { ok = false; break; }
-                    tc::fence_after_sync();
-                    const uint32_t sa = dme::smem_addr(smem + r.stage * Sh::STAGE_BYTES);
-                    const uint64_t ad = tc::smem_desc_sw128(sa, 16, 1024);
-                    const uint64_t bd = tc::smem_desc_sw128(sa + Sh::A_BYTES, 16, 1024);
+                const uint64_t ad = a0 + uint64_t(r.stage * (Sh::STAGE_BYTES / 16)), bd = ad + uint64_t(Sh::A_BYTES / 16);
+                if (tc::elect_one()) {
                     #pragma unroll
                     for (int ks = 0; ks < kTK / 16; ++ks)
-                        tc::mma_ss(tmem + b * 256, ad + uint64_t(ks * 2), bd + uint64_t(ks * 2), idesc, (kb | ks) != 0);
+                        tc::mma_ss(tm + b * 256, ad + uint64_t(ks * 2), bd + uint64_t(ks * 2), idesc, (kb | ks) != 0);
                     tc::commit(&empty[r.stage]);
-                    r.advance();
+                    if (kb == kblocks - 1) tc::commit(&acc_full[b]);
                 }
-                if (!ok) break;
-                tc::commit(&acc_full[b]);
+                __syncwarp();
+                r.advance();
             }
         }
     } else {

@@ -258,86 +258,109 @@ prefill_tc_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap map
         }
       } else if (warp == kMmaWarp) {
         // ---------------------------------- MMA issuer ------------------------------------
-        if (lane == 0) {
-            constexpr uint32_t idesc_qk = tc::instr_desc_f16(kBM, kBN, Fmt<T>::id, 0, 0);
-            constexpr uint32_t idesc_pv = tc::instr_desc_f16(kBM, DV, Fmt<T>::id, 0, 1);
-            // Descriptors differ from a per-tile base only in the 14-bit start-address field
-            // (units of 16 bytes), so a k-step is one integer add of a compile-time constant on the base;
-            // the k loops are unrolled so that the issue overhead per MMA stays far below its 64 cycles.
-            const uint64_t q_base = tc::smem_desc_sw128(sm_q, 16, 1024);
-            const uint64_t k_base = tc::smem_desc_sw128(sm_k, 16, 1024);
-            const uint64_t v_base = tc::smem_desc_sw128(sm_v, Sh::SUB_BYTES, 1024);
-            auto issue_qk = [&](int t, int kstage) {
-                const uint64_t qd = q_base + uint64_t((t * Sh::QK_BYTES) >> 4);
-                const uint64_t kd = k_base + uint64_t((kstage * Sh::QK_BYTES) >> 4);
-                #pragma unroll
-                for (int ks = 0; ks < Sh::QK_SUB * 4; ++ks) {
-                    const uint32_t off16 = (uint32_t(ks >> 2) * Sh::SUB_BYTES + uint32_t(ks & 3) * 32u) >> 4;
-                    tc::mma_ss(tmem + t * kBN, qd + off16, kd + off16, idesc_qk, ks > 0);
-                }
-            };
-            auto issue_pv = [&](int t, int vstage, bool first, int kk0, int kk1) {  // 16-key steps kk0 .. kk1-1 of the tile
-                const uint64_t vd = v_base + uint64_t((vstage * Sh::V_BYTES) >> 4);
-                #pragma unroll
-                for (int kk = kk0; kk < kk1; ++kk)
-                    tc::mma_ts(tmem + 256 + t * 128, tmem + t * kBN + kk * 8, vd + uint64_t(kk * (2048 >> 4)),
-                               idesc_pv, !(first && kk == 0));
-            };
-            dme::Ring<KST> kr; dme::Ring<VST> vr;
-            int cs0 = 0, cs1 = 0;          // steps of tile 0 / 1 in earlier items: phase of s_full / p_half
-            int co0 = 0, co1 = 0;          // earlier items in which the tile had work: phase of o_done / o_free
-            bool ok = true;
-            for (int it = 0; ok; ++it) {
-                const int id = next_item(it);
-                if (id < 0) { ok = id != -2; break; }
-                const PrefillItem w = prefill_item<Sh>(p, id);
-                const int nmax = w.nmax, n0 = w.n[0], n1 = w.n[1];
-                ok = dme::wait(q_full, uint32_t(it & 1), p.status);
-                if (ok) ok = dme::wait(&k_full[kr.stage], kr.phase, p.status);
-                if (!ok) break;
-                tc::fence_after_sync();
+        // All lanes walk the loops and wait; one issues (tc::elect_one).  What the loops branch on is made warp-uniform by a
+        // shuffle, so that descriptors and ring state live in uniform registers.
+        constexpr uint32_t idesc_qk = tc::instr_desc_f16(kBM, kBN, Fmt<T>::id, 0, 0);
+        constexpr uint32_t idesc_pv = tc::instr_desc_f16(kBM, DV, Fmt<T>::id, 0, 1);
+        // Descriptors differ from a per-tile base only in the 14-bit start-address field
+        // (units of 16 bytes), so a k-step is one integer add of a compile-time constant on the base;
+        // the k loops are unrolled so that the issue overhead per MMA stays far below its 64 cycles.
+        const uint64_t q_base = tc::smem_desc_sw128(sm_q, 16, 1024);
+        const uint64_t k_base = tc::smem_desc_sw128(sm_k, 16, 1024);
+        const uint64_t v_base = tc::smem_desc_sw128(sm_v, Sh::SUB_BYTES, 1024);
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, dme::wait(bar, parity, p.status)) != 0; };
+        auto issue_qk = [&](int t, int kstage) {
+            const uint64_t qd = q_base + uint64_t((t * Sh::QK_BYTES) >> 4);
+            const uint64_t kd = k_base + uint64_t((kstage * Sh::QK_BYTES) >> 4);
+            #pragma unroll
+            for (int ks = 0; ks < Sh::QK_SUB * 4; ++ks) {
+                const uint32_t off16 = (uint32_t(ks >> 2) * Sh::SUB_BYTES + uint32_t(ks & 3) * 32u) >> 4;
+                tc::mma_ss(tm + t * kBN, qd + off16, kd + off16, idesc_qk, ks > 0);
+            }
+        };
+        auto issue_pv = [&](int t, int vstage, bool first, int kk0, int kk1) {  // 16-key steps kk0 .. kk1-1 of the tile
+            const uint64_t vd = v_base + uint64_t((vstage * Sh::V_BYTES) >> 4);
+            #pragma unroll
+            for (int kk = kk0; kk < kk1; ++kk)
+                tc::mma_ts(tm + 256 + t * 128, tm + t * kBN + kk * 8, vd + uint64_t(kk * (2048 >> 4)),
+                           idesc_pv, !(first && kk == 0));
+        };
+        dme::Ring<KST> kr; dme::Ring<VST> vr;
+        int cs0 = 0, cs1 = 0;          // steps of tile 0 / 1 in earlier items: phase of s_full / p_half
+        int co0 = 0, co1 = 0;          // earlier items in which the tile had work: phase of o_done / o_free
+        bool ok = true;
+        for (int it = 0; ok; ++it) {
+            if (!wait(&item_full[it & 1], uint32_t((it >> 1) & 1))) { ok = false; break; }
+            const int id = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&s_item[it & 1]), 0);
+            if (tc::elect_one()) dme::mbar_arrive(&item_empty[it & 1]);
+            __syncwarp();
+            if (id < 0) break;
+            const PrefillItem w = prefill_item<Sh>(p, id);
+            const int nmax = w.nmax, n0 = w.n[0], n1 = w.n[1];
+            ok = wait(q_full, uint32_t(it & 1)) && wait(&k_full[kr.stage], kr.phase);
+            if (!ok) break;
+            tc::fence_after_sync();
+            if (tc::elect_one()) {
                 if (n0 > 0) { issue_qk(0, kr.stage); tc::commit(&s_full[0]); }
                 if (n1 > 0) { issue_qk(1, kr.stage); tc::commit(&s_full[1]); }
                 tc::commit(&k_empty[kr.stage]);
-                kr.advance();
                 if (nmax == 1) tc::commit(q_empty);
-                // one tile's share of step j: P.V over the two halves of P as they arrive, then the next Q.K^T
-                auto tile_step = [&](auto tc_t, int j, int nt, int cst, int cot) -> bool {
-                    constexpr int t = decltype(tc_t)::value;
-                    if (j >= nt) return true;
-                    if (!dme::wait(&p_half[2 * t], uint32_t((cst + j) & 1), p.status)) return false;
-                    // the first P.V of an item overwrites O_t: the previous item's epilogue must have read it
-                    if (j == 0 && cot > 0 && !dme::wait(&o_free[t], uint32_t((cot - 1) & 1), p.status)) return false;
+            }
+            __syncwarp();
+            kr.advance();
+            // one tile's share of step j: P.V over the two halves of P as they arrive, then the next Q.K^T
+            auto tile_step = [&](auto tc_t, int j, int nt, int cst, int cot) -> bool {
+                constexpr int t = decltype(tc_t)::value;
+                if (j >= nt) return true;
+                if (!wait(&p_half[2 * t], uint32_t((cst + j) & 1))) return false;
+                // the first P.V of an item overwrites O_t: the previous item's epilogue must have read it
+                if (j == 0 && cot > 0 && !wait(&o_free[t], uint32_t((cot - 1) & 1))) return false;
+                tc::fence_after_sync();
+                if (tc::elect_one()) issue_pv(t, vr.stage, j == 0, 0, 2 * kFirstChunks);   // the first hand-off's keys while the softmax finishes the rest
+                __syncwarp();
+                if (!wait(&p_half[2 * t + 1], uint32_t((cst + j) & 1))) return false;
+                // (with one K stage the next keys arrive while this step's softmax runs: waited for only here, after P.V is issued)
+                if (!LATENT || j + 1 >= nt) {
                     tc::fence_after_sync();
-                    issue_pv(t, vr.stage, j == 0, 0, 2 * kFirstChunks);   // the first hand-off's keys while the softmax finishes the rest
-                    if (!dme::wait(&p_half[2 * t + 1], uint32_t((cst + j) & 1), p.status)) return false;
-                    tc::fence_after_sync();
-                    issue_pv(t, vr.stage, j == 0, 2 * kFirstChunks, kBN / 16);
-                    // (with one K stage the next keys arrive while this step's softmax runs: waited for only here)
-                    if (LATENT && j + 1 < nt && !dme::wait(&k_full[kr.stage], kr.phase, p.status)) return false;
-                    if (LATENT) tc::fence_after_sync();
-                    if (j + 1 < nt) { issue_qk(t, kr.stage); tc::commit(&s_full[t]); }
-                    else tc::commit(&o_done[t]);
+                    if (tc::elect_one()) {
+                        issue_pv(t, vr.stage, j == 0, 2 * kFirstChunks, kBN / 16);
+                        if (j + 1 < nt) { issue_qk(t, kr.stage); tc::commit(&s_full[t]); }
+                        else tc::commit(&o_done[t]);
+                    }
+                    __syncwarp();
                     return true;
-                };
-                for (int j = 0; j < nmax && ok; ++j) {
-                    ok = dme::wait(&v_full[vr.stage], vr.phase, p.status);
-                    if (!LATENT && ok && j + 1 < nmax) ok = dme::wait(&k_full[kr.stage], kr.phase, p.status);
-                    if (!ok) break;
-                    ok = tile_step(std::integral_constant<int, 0>{}, j, n0, cs0, co0);
-                    if (ok) ok = tile_step(std::integral_constant<int, 1>{}, j, n1, cs1, co1);
-                    if (!ok) break;
+                }
+                tc::fence_after_sync();
+                if (tc::elect_one()) issue_pv(t, vr.stage, j == 0, 2 * kFirstChunks, kBN / 16);
+                __syncwarp();
+                if (!wait(&k_full[kr.stage], kr.phase)) return false;
+                tc::fence_after_sync();
+                if (tc::elect_one()) { issue_qk(t, kr.stage); tc::commit(&s_full[t]); }
+                __syncwarp();
+                return true;
+            };
+            for (int j = 0; j < nmax && ok; ++j) {
+                ok = wait(&v_full[vr.stage], vr.phase);
+                if (!LATENT && ok && j + 1 < nmax) ok = wait(&k_full[kr.stage], kr.phase);
+                if (!ok) break;
+                ok = tile_step(std::integral_constant<int, 0>{}, j, n0, cs0, co0);
+                if (ok) ok = tile_step(std::integral_constant<int, 1>{}, j, n1, cs1, co1);
+                if (!ok) break;
+                if (tc::elect_one()) {
                     tc::commit(&v_empty[vr.stage]);
-                    vr.advance();
                     if (j + 1 < nmax) {
-                        tc::commit(&k_empty[kr.stage]); kr.advance();
+                        tc::commit(&k_empty[kr.stage]);
                         if (j + 2 == nmax) tc::commit(q_empty);           // that was the item's last Q.K^T
                     }
                 }
-                cs0 += n0; cs1 += n1; co0 += n0 > 0; co1 += n1 > 0;
+                __syncwarp();
+                vr.advance();
+                if (j + 1 < nmax) kr.advance();
             }
-            if (!ok) atomicExch(&s_failed, 1);
+            cs0 += n0; cs1 += n1; co0 += n0 > 0; co1 += n1 > 0;
         }
+        if (!ok && lane == 0) atomicExch(&s_failed, 1);
       }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");

@@ -24,7 +24,7 @@ enum Knob {
     KNOB_DECODE_SPLITS,         // split-KV count override
     KNOB_DECODE_FUSED_COMBINE,  // 1: the tensor-core decode kernel merges its splits itself, 0: separate combine launch
     KNOB_DECODE_VARIANT,        // 1: tensor-map + mma.sync kernel, 0: bulk-copy + vector kernel
-    KNOB_PREFILL_VARIANT,
+    KNOB_PREFILL_VARIANT,       // bit 1: one CTA per work item; bit 4: forced items, bit 2: of one tile, bit 3: heads of a group packed
     KNOB_RUNTIME_GRAPH,         // 1: the runtime replays its decode step as a CUDA graph, 0: launches it every step
     KNOB_RUNTIME_PDL,           // 1: skinny kernels launch as programmatic dependents (weights prefetched before the wait)
     KNOB_RUNTIME_ROPE_FUSED,    // 1: RoPE + KV scatter in the Q/K/V projection's epilogue, 0: separate kernel

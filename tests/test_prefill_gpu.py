@@ -166,3 +166,28 @@ def test_launches_on_two_streams_do_not_share_a_work_counter(b200p, torch_cuda):
     for oa, ob in outs:
         assert torch.equal(oa, ref_a) and torch.equal(ob, ref_b)
     assert b200p.device_status() == 0
+
+
+# rows that end inside, at and just past a tile and a pair of tiles; runs of rows that wrap to the next head inside a tile; one
+# row per head; fewer and more items than SMs; keys of one tile and of many
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("batch,heads,kv,S", [(1, 4, 1, 1), (2, 8, 2, 20), (1, 8, 1, 127), (1, 4, 4, 128), (3, 8, 2, 129), (1, 6, 2, 255), (2, 4, 1, 257), (1, 8, 4, 385), (2, 32, 4, 555), (1, 8, 8, 700)])
+def test_work_items_of_every_form_give_the_same_bits(b200p, torch_cuda, D, causal, batch, heads, kv, S):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(S * 7 + heads)
+    q, k, v = (torch.randn((batch, h, S, D), device="cuda", generator=g).bfloat16() for h in (heads, kv, kv))
+    outs = []
+    try:
+        for variant in (16, 20, 24, 28, -1):                     # pairs, single tiles, both packed, the rule's choice
+            b200p.set_tuning("prefill_variant", variant)
+            outs.append(b200p.prefill(q, k, v, causal=causal))
+    finally:
+        b200p.set_tuning("prefill_variant", -1)
+    for o in outs[1:]:
+        assert torch.equal(o, outs[0])
+    qd, kd, vd = q.double(), k.double().repeat_interleave(heads // kv, 1), v.double().repeat_interleave(heads // kv, 1)
+    s = qd @ kd.transpose(-1, -2) * D ** -0.5
+    if causal:
+        s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    assert (outs[0].double() - s.softmax(-1) @ vd).abs().max() < 2e-2

@@ -6,20 +6,20 @@
 //   step 1  fa_dpp    research/flash-attention-mi300x/fa_dpp.hip:52-167
 //           the same with wave::dpp::reduce_max_bcast / reduce_sum_bcast
 //   step 2  fa_dme    research/flash-attention-mi300x/fa_dme.hip:74-221
-//           step 1 + K/V tiles double-buffered by asynchronous copies
+//           step 1 + K/V tiles double-buffered by asynchronous copies (cp.async)
 //   (step 3, fa_mfma2, is the tcgen05 kernel in prefill.cu)
 // and, with fp32 I/O, the reference's fp32 kernels
 //   research/flash-attention-mi300x/kernels/fa_naive.hip:118-278
 //   research/flash-attention-mi300x/kernels/fa_dpp.hip:167-313
 // whose launch takes (seq_len, n_heads, scale).
 //
-// Tiling is the reference's: Br = 16 query rows per CTA (one warp per row),
+// Tiling is the reference's: Br = 16 query rows per CTA (two per warp),
 // Bc = 64 keys per tile.  A 64-key score row is held by ONE 32-lane warp as an
 // adjacent pair per lane (keys 2l, 2l+1), which is exactly the shape the pair
 // overloads of wave64.cuh reduce; O stays in registers (D/32 dims per lane)
 // instead of the reference's LDS accumulator.
 // These kernels exist for parity with the reference's steps and to exercise the
-// primitives and the TMA ring in a simple setting; at the reference's config
+// primitives in a simple setting; at the reference's config
 // (0.54 GFLOP, 4 MiB) they are launch-bound on a B200.
 // ---------------------------------------------------------------------------
 #include "common.cuh"
@@ -49,135 +49,161 @@ template <> __device__ __forceinline__ float exp_for<float>(float x)         { r
 template <> __device__ __forceinline__ float exp_for<__half>(float x)        { return __expf(x); }
 template <> __device__ __forceinline__ float exp_for<__nv_bfloat16>(float x) { return __expf(x); }
 
+// What bounds this kernel is shared memory: a warp with one row reads the whole K and V tile for it, and q again for every
+// lane (40 KB per row and tile).  Here two rows share each read, and every lane reads its own two key rows at the same
+// 16-byte chunk, so q is a broadcast; the keys lie 16 bytes further apart than their size, odd keys behind the even ones, and
+// the eight lanes of a shared-memory phase hit eight different bank groups.  (Four rows per warp read less but leave too
+// few warps: within 10 % at 8 heads x 512 keys either way.)  Before and after: 8 heads of 64, 512 keys, fp32, step 1
+// 57.7 -> 38.0 us, step 2 54.6 -> 34.6 (its copies were bulk copies behind an mbarrier and an abort word to clear); 12 heads, 333 keys,
+// fp32, which went to the one-row kernels: 110.6 -> 29.2; 24 heads of 128, 1024 keys, fp16: 675 -> 505.
+// Lengths need not be multiples of the tiles: keys past the end get no weight, rows past the end are not stored.
+constexpr int kRowsPerWarp = 2, kStepThreads = kBr / kRowsPerWarp * 32;
+template <typename T, int D> struct StepTile {
+    static constexpr int ROW = D * int(sizeof(T));                         // bytes of a key
+    static constexpr int KROW = ROW + 16;                                  // between two slots of K
+    static constexpr int K_BYTES = kBc * KROW, V_BYTES = kBc * ROW;
+};
+
 template <typename T, int D, int STEP>
-__global__ void __launch_bounds__(kBr * 32)
+__global__ void __launch_bounds__(kStepThreads)
 fa_step_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V, T* __restrict__ O,
-               int seq_q, int seq_k, int heads, float scale, int* abort_word, int* sticky) {
+               int seq_q, int seq_k, int heads, float scale, float m_first) {
+    using Sh = StepTile<T, D>;
     constexpr int DPL = D / 32;                           // output dims per lane
-    constexpr uint32_t kTileBytes = kBc * D * sizeof(T);
+    constexpr int NB = STEP == 2 ? 2 : 1;                 // tile buffers
+    constexpr int R = kRowsPerWarp;
     extern __shared__ __align__(128) unsigned char smem[];
-    T* Kt = reinterpret_cast<T*>(smem);                                    // [2][Bc*D] (one buffer used for STEP < 2)
-    T* Vt = reinterpret_cast<T*>(smem + 2 * kTileBytes);
-    float* prow = reinterpret_cast<float*>(smem + 4 * kTileBytes);         // [Br][Bc]
+    unsigned char* Kt = smem;                                              // [NB][kBc slots][KROW]: key k in slot (k % 2) * 32 + k / 2
+    unsigned char* Vt = smem + NB * Sh::K_BYTES;                           // [NB][kBc][D]
+    float* prow = reinterpret_cast<float*>(Vt + NB * Sh::V_BYTES);         // [Br][Bc]
     float* qs = prow + kBr * kBc;                                          // [Br][D]
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + 4 * kTileBytes + (kBr * kBc + kBr * D) * sizeof(float));
-    __shared__ int s_failed;
 
     // blockIdx.x = batch * heads * (seq_q/Br) + head * (seq_q/Br) + qblk   (fa_naive.hip:70-71)
-    const int qblocks = seq_q / kBr;
+    const int qblocks = (seq_q + kBr - 1) / kBr;
     const int qblk = blockIdx.x % qblocks;
     const int bh = blockIdx.x / qblocks;                                   // batch * heads + head
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const T* Qrow = Q + (size_t(bh) * seq_q + qblk * kBr + warp) * D;
+    const int row0 = qblk * kBr + warp * R;                                // this warp's first query row
     const T* Kb = K + size_t(bh) * seq_k * D;
     const T* Vb = V + size_t(bh) * seq_k * D;
-    T* Orow = O + (size_t(bh) * seq_q + qblk * kBr + warp) * D;
-    const int ntiles = seq_k / kBc;
+    const int ntiles = (seq_k + kBc - 1) / kBc;
 
-    if (STEP == 2 && threadIdx.x == 0) {
-        s_failed = 0;
-        dme::mbar_init(&full[0], 1); dme::mbar_init(&full[1], 1);
-        dme::mbar_init_fence();
-    }
-    // This warp's query row as fp32.  With 16-bit keys a lane reads 8 floats of q per 16-byte key chunk, so the eight
-    // lanes of a shared-memory phase read pieces 32 bytes apart, 256 bytes in all: pieces 0 and 4 would share their
-    // banks.  The row is therefore stored with its float4 index f at f ^ ((f >> 3) & 1).
-    constexpr bool kSwizzleQ = sizeof(T) == 2;
-    auto qpos = [](int f4) -> int { return kSwizzleQ ? (f4 ^ ((f4 >> 3) & 1)) : f4; };
-    float* q = qs + warp * D;
-    for (int d = lane; d < D; d += 32) q[qpos(d / 4) * 4 + d % 4] = to_float(Qrow[d]);
-    __syncthreads();
-    if (STEP == 2 && threadIdx.x == 0) {                  // prologue: tile 0 -> buffer 0
-        dme::mbar_arrive_expect_tx(&full[0], 2 * kTileBytes);
-        dme::copy_tile_1d(Kt, Kb, kTileBytes, &full[0]);
-        dme::copy_tile_1d(Vt, Vb, kTileBytes, &full[0]);
-    }
-
-    float m = -1e38f, l = 0.f;                            // the reference's initial running max
-    float o[DPL];
+    float* q = qs + warp * R * D;
     #pragma unroll
-    for (int i = 0; i < DPL; ++i) o[i] = 0.f;
-    bool ok = true;
+    for (int r = 0; r < R; ++r)
+        for (int d = lane; d < D; d += 32) q[r * D + d] = row0 + r < seq_q ? to_float(Q[(size_t(bh) * seq_q + row0 + r) * D + d]) : 0.f;
+    __syncwarp();
+    // tile j into buffer j & 1, 16 bytes per thread per step: asynchronous copies (step 2), or through registers
+    auto copy_tile = [&](int j) {
+        constexpr int CPR = Sh::ROW / 16;                                 // chunks per key
+        const int nb = STEP == 2 ? (j & 1) : 0, n = min(kBc, seq_k - j * kBc);
+        const uint4* ks = reinterpret_cast<const uint4*>(Kb + size_t(j) * kBc * D);
+        const uint4* vs = reinterpret_cast<const uint4*>(Vb + size_t(j) * kBc * D);
+        unsigned char* kd = Kt + nb * Sh::K_BYTES;
+        unsigned char* vd = Vt + nb * Sh::V_BYTES;
+        for (int i = threadIdx.x; i < n * CPR; i += kStepThreads) {
+            const int k = i / CPR, c = i % CPR;
+            unsigned char* kslot = kd + ((k & 1) * 32 + (k >> 1)) * Sh::KROW + c * 16;
+            if (STEP == 2) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dme::smem_addr(kslot)), "l"(ks + i) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dme::smem_addr(vd + i * 16)), "l"(vs + i) : "memory");
+            } else {
+                *reinterpret_cast<uint4*>(kslot) = ks[i];
+                reinterpret_cast<uint4*>(vd)[i] = vs[i];
+            }
+        }
+        if (STEP == 2) asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (STEP == 2) copy_tile(0);
+
+    float m[R], l[R], o[R][DPL];
+    #pragma unroll
+    for (int r = 0; r < R; ++r) {
+        m[r] = m_first; l[r] = 0.f;
+        #pragma unroll
+        for (int i = 0; i < DPL; ++i) o[r][i] = 0.f;
+    }
 
     for (int j = 0; j < ntiles; ++j) {
-        const int buf = (STEP == 2) ? (j & 1) : 0;
-        const T* Kc = Kt + buf * kBc * D;
-        const T* Vc = Vt + buf * kBc * D;
-        if (STEP == 2) {
-            if (threadIdx.x == 0 && j + 1 < ntiles) {     // prefetch tile j+1 into the other buffer
-                const int nb = (j + 1) & 1;
-                dme::mbar_arrive_expect_tx(&full[nb], 2 * kTileBytes);
-                dme::copy_tile_1d(Kt + nb * kBc * D, Kb + size_t(j + 1) * kBc * D, kTileBytes, &full[nb]);
-                dme::copy_tile_1d(Vt + nb * kBc * D, Vb + size_t(j + 1) * kBc * D, kTileBytes, &full[nb]);
-            }
-            if (!dme::wait(&full[buf], uint32_t(j >> 1) & 1u, abort_word)) { ok = false; }
-        } else {
-            // cooperative synchronous tile load, 16 bytes per thread per step
-            const uint4* ks = reinterpret_cast<const uint4*>(Kb + size_t(j) * kBc * D);
-            const uint4* vs = reinterpret_cast<const uint4*>(Vb + size_t(j) * kBc * D);
-            uint4* kd = reinterpret_cast<uint4*>(Kt);
-            uint4* vd = reinterpret_cast<uint4*>(Vt);
-            for (int i = threadIdx.x; i < int(kTileBytes / 16); i += kBr * 32) { kd[i] = ks[i]; vd[i] = vs[i]; }
-            __syncthreads();
-        }
-        // S[row][2l], S[row][2l+1].  Every lane reads its own two key rows, which lie a multiple of 128 bytes apart:
-        // read in the same order they would all hit the same banks.  Lane l starts at 16-byte chunk l of its rows and
-        // wraps, so the eight lanes of a shared-memory phase read eight different chunks (and eight different pieces of q).
-        float s0 = 0.f, s1 = 0.f;
+        const int buf = STEP == 2 ? (j & 1) : 0, live = min(kBc, seq_k - j * kBc);
+        const unsigned char* Kc = Kt + buf * Sh::K_BYTES;
+        unsigned char* Vc = Vt + buf * Sh::V_BYTES;
+        if (STEP == 2) {                                                   // prefetch tile j + 1, wait for tile j
+            if (j + 1 < ntiles) { copy_tile(j + 1); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+            else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        } else copy_tile(j);
+        if (live < kBc)                                                    // no weight times whatever was there must be nothing
+            for (int i = live * (Sh::ROW / 16) + threadIdx.x; i < kBc * (Sh::ROW / 16); i += kStepThreads) reinterpret_cast<uint4*>(Vc)[i] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
+        // S[row][2l], S[row][2l+1]
+        float s0[R], s1[R];
+        #pragma unroll
+        for (int r = 0; r < R; ++r) s0[r] = s1[r] = 0.f;
         {
-            constexpr int EPC = 16 / int(sizeof(T)), NCH = D / EPC;           // elements per chunk, chunks per row
-            const uint4* kr0 = reinterpret_cast<const uint4*>(Kc + (2 * lane) * D);
-            const uint4* kr1 = kr0 + NCH;
-            #pragma unroll
+            constexpr int EPC = 16 / int(sizeof(T)), NCH = D / EPC;       // elements per chunk, chunks per row
+            const uint4* kr0 = reinterpret_cast<const uint4*>(Kc + lane * Sh::KROW);
+            const uint4* kr1 = reinterpret_cast<const uint4*>(Kc + (32 + lane) * Sh::KROW);
+            #pragma unroll 4
             for (int c = 0; c < NCH; ++c) {
-                const int cc = (c + lane) & (NCH - 1);
-                const uint4 ka = kr0[cc], kb = kr1[cc];
+                const uint4 ka = kr0[c], kb = kr1[c];
                 const T* ea = reinterpret_cast<const T*>(&ka);
                 const T* eb = reinterpret_cast<const T*>(&kb);
-                float qv[EPC];
                 #pragma unroll
-                for (int e = 0; e < EPC; e += 4) *reinterpret_cast<float4*>(&qv[e]) = *reinterpret_cast<const float4*>(q + qpos((cc * EPC + e) / 4) * 4);
-                #pragma unroll
-                for (int e = 0; e < EPC; ++e) { s0 = fmaf(qv[e], to_float(ea[e]), s0); s1 = fmaf(qv[e], to_float(eb[e]), s1); }
+                for (int r = 0; r < R; ++r) {
+                    float qv[EPC];
+                    #pragma unroll
+                    for (int e = 0; e < EPC; e += 4) *reinterpret_cast<float4*>(&qv[e]) = *reinterpret_cast<const float4*>(q + r * D + c * EPC + e);
+                    #pragma unroll
+                    for (int e = 0; e < EPC; ++e) { s0[r] = fmaf(qv[e], to_float(ea[e]), s0[r]); s1[r] = fmaf(qv[e], to_float(eb[e]), s1[r]); }
+                }
             }
         }
-        s0 *= scale; s1 *= scale;
         // online softmax (cdna3-prims/examples/fused_softmax.hpp:38-48)
-        float rmax, rsum;
-        if (STEP == 0) rmax = portable_reduce_bcast(s0, s1, wave::MaxOp{});
-        else           rmax = wave::dpp::reduce_max_bcast(s0, s1);
-        const float m_new = fmaxf(m, rmax);
-        const float p0 = exp_for<T>(s0 - m_new), p1 = exp_for<T>(s1 - m_new);
-        if (STEP == 0) rsum = portable_reduce_bcast(p0, p1, wave::SumOp{});
-        else           rsum = wave::dpp::reduce_sum_bcast(p0, p1);
-        const float resc = exp_for<T>(m - m_new);
-        l = resc * l + rsum;
-        m = m_new;
         #pragma unroll
-        for (int i = 0; i < DPL; ++i) o[i] *= resc;
-        // O[row][d] += sum_k P[row][k] * V[k][d]
-        prow[warp * kBc + 2 * lane] = p0;
-        prow[warp * kBc + 2 * lane + 1] = p1;
+        for (int r = 0; r < R; ++r) {
+            constexpr float kLowest = -3.402823466e+38f;
+            s0[r] = 2 * lane < live ? s0[r] * scale : kLowest;
+            s1[r] = 2 * lane + 1 < live ? s1[r] * scale : kLowest;
+            const float rmax = STEP == 0 ? portable_reduce_bcast(s0[r], s1[r], wave::MaxOp{}) : wave::dpp::reduce_max_bcast(s0[r], s1[r]);
+            const float m_new = fmaxf(m[r], rmax);
+            const float p0 = 2 * lane < live ? exp_for<T>(s0[r] - m_new) : 0.f, p1 = 2 * lane + 1 < live ? exp_for<T>(s1[r] - m_new) : 0.f;
+            const float rsum = STEP == 0 ? portable_reduce_bcast(p0, p1, wave::SumOp{}) : wave::dpp::reduce_sum_bcast(p0, p1);
+            const float resc = exp_for<T>(m[r] - m_new);
+            l[r] = resc * l[r] + rsum;
+            m[r] = m_new;
+            #pragma unroll
+            for (int i = 0; i < DPL; ++i) o[r][i] *= resc;
+            *reinterpret_cast<float2*>(&prow[(warp * R + r) * kBc + 2 * lane]) = make_float2(p0, p1);
+        }
         __syncwarp();
-        #pragma unroll 4
+        // O[row][d] += sum_k P[row][k] * V[k][d]
+        #pragma unroll 2
         for (int k = 0; k < kBc; k += 4) {
-            const float4 p4 = *reinterpret_cast<const float4*>(&prow[warp * kBc + k]);      // broadcast read
-            const float pk[4] = {p4.x, p4.y, p4.z, p4.w};
+            float4 p4[R];
+            #pragma unroll
+            for (int r = 0; r < R; ++r) p4[r] = *reinterpret_cast<const float4*>(&prow[(warp * R + r) * kBc + k]);      // broadcast reads
             #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
+                float v[DPL];
                 #pragma unroll
-                for (int i = 0; i < DPL; ++i) o[i] = fmaf(pk[kk], to_float(Vc[(k + kk) * D + lane * DPL + i]), o[i]);
+                for (int i = 0; i < DPL; ++i) v[i] = to_float(reinterpret_cast<const T*>(Vc)[(k + kk) * D + lane * DPL + i]);
+                #pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const float pk = kk == 0 ? p4[r].x : kk == 1 ? p4[r].y : kk == 2 ? p4[r].z : p4[r].w;
+                    #pragma unroll
+                    for (int i = 0; i < DPL; ++i) o[r][i] = fmaf(pk, v[i], o[r][i]);
+                }
             }
         }
         __syncthreads();                                  // tile buffers and prow are reused next iteration
     }
-    const float inv = l > 0.f ? 1.f / l : 0.f;            // kernels/fa_naive.hip: l_inv = l > 0 ? 1/l : 0
     #pragma unroll
-    for (int i = 0; i < DPL; ++i) Orow[lane * DPL + i] = from_float<T>(o[i] * inv);
-    if (STEP == 2) {
-        if (!ok) atomicExch(&s_failed, 1);
-        __syncthreads();
-        if (threadIdx.x == 0 && s_failed) atomicExch(sticky, 1);
+    for (int r = 0; r < R; ++r) {
+        const float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;  // kernels/fa_naive.hip: l_inv = l > 0 ? 1/l : 0
+        if (row0 + r < seq_q) {
+            #pragma unroll
+            for (int i = 0; i < DPL; ++i) O[(size_t(bh) * seq_q + row0 + r) * D + lane * DPL + i] = from_float<T>(o[r][i] * inv);
+        }
     }
 }
 
@@ -308,37 +334,34 @@ int launch_rows_bc(int bc, bool dpp, const float* Q, const float* K, const float
 
 template <typename T, int D, int STEP>
 int launch_step(const void* Q, const void* K, const void* V, void* O, int batch, int heads, int seq_q, int seq_k,
-                float scale, cudaStream_t st) {
-    const size_t smem = 4 * size_t(kBc) * D * sizeof(T) + (kBr * kBc + kBr * D) * sizeof(float) + 64;
-    int* sticky = device_status_ptr();
-    if (!sticky) return B200P_E_NO_DEVICE;
-    LaunchSlot slot{};                                         // the launch's own abort word (only the async step waits)
-    if (STEP == 2) { if (int se = take_launch_slot(st, &slot)) return se; }
+                float scale, float m_first, cudaStream_t st) {
+    using Sh = StepTile<T, D>;
+    const size_t smem = size_t(STEP == 2 ? 2 : 1) * (Sh::K_BYTES + Sh::V_BYTES) + (kBr * kBc + kBr * D) * sizeof(float);
     auto kern = fa_step_kernel<T, D, STEP>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return int(e);
     }
-    const unsigned grid = unsigned(batch) * heads * (seq_q / kBr);
-    kern<<<grid, kBr * 32, smem, st>>>(static_cast<const T*>(Q), static_cast<const T*>(K), static_cast<const T*>(V),
-                                       static_cast<T*>(O), seq_q, seq_k, heads, scale, slot.abort, sticky);
+    const unsigned grid = unsigned(batch) * heads * ((seq_q + kBr - 1) / kBr);
+    kern<<<grid, kStepThreads, smem, st>>>(static_cast<const T*>(Q), static_cast<const T*>(K), static_cast<const T*>(V),
+                                       static_cast<T*>(O), seq_q, seq_k, heads, scale, m_first);
     return launched();
 }
 template <typename T, int D>
 int launch_step_s(int step, const void* Q, const void* K, const void* V, void* O, int batch, int heads, int seq_q,
-                  int seq_k, float scale, cudaStream_t st) {
+                  int seq_k, float scale, float m_first, cudaStream_t st) {
     switch (step) {
-        case 0: return launch_step<T, D, 0>(Q, K, V, O, batch, heads, seq_q, seq_k, scale, st);
-        case 1: return launch_step<T, D, 1>(Q, K, V, O, batch, heads, seq_q, seq_k, scale, st);
-        case 2: return launch_step<T, D, 2>(Q, K, V, O, batch, heads, seq_q, seq_k, scale, st);
+        case 0: return launch_step<T, D, 0>(Q, K, V, O, batch, heads, seq_q, seq_k, scale, m_first, st);
+        case 1: return launch_step<T, D, 1>(Q, K, V, O, batch, heads, seq_q, seq_k, scale, m_first, st);
+        case 2: return launch_step<T, D, 2>(Q, K, V, O, batch, heads, seq_q, seq_k, scale, m_first, st);
     }
     return B200P_E_OP;
 }
 template <typename T>
 int launch_step_d(int step, int D, const void* Q, const void* K, const void* V, void* O, int batch, int heads,
-                  int seq_q, int seq_k, float scale, cudaStream_t st) {
-    return D == 64 ? launch_step_s<T, 64>(step, Q, K, V, O, batch, heads, seq_q, seq_k, scale, st)
-                   : launch_step_s<T, 128>(step, Q, K, V, O, batch, heads, seq_q, seq_k, scale, st);
+                  int seq_q, int seq_k, float scale, float m_first, cudaStream_t st) {
+    return D == 64 ? launch_step_s<T, 64>(step, Q, K, V, O, batch, heads, seq_q, seq_k, scale, m_first, st)
+                   : launch_step_s<T, 128>(step, Q, K, V, O, batch, heads, seq_q, seq_k, scale, m_first, st);
 }
 
 } // namespace
@@ -380,16 +403,18 @@ extern "C" int b200p_fa_step(int step, int dtype, const void* Q, const void* K, 
     }
     if (sm_count() <= 0) return B200P_E_NO_DEVICE;
     if (scale == 0.f) scale = 1.f / sqrtf(float(D));
+    float m_first = -1e38f;                                // the reference's initial running max
     if (seq_q % kBr != 0 || seq_k % kBc != 0) {
-        // Lengths off the Br = 16 / Bc = 64 tiling: the fp32-I/O kernels take any seq_len by padding the
-        // keys past the end (kernels/fa_naive.hip:158-169); the 16-bit step kernels keep the reference's tiling.
+        // Lengths off the Br = 16 / Bc = 64 tiling: fp32 I/O takes any seq_len like the reference's fp32 kernels, whose running
+        // max starts at the lowest float (kernels/fa_naive.hip:158-169); the 16-bit steps keep the reference's tiling.
         if (dtype != B200P_F32 || seq_q != seq_k) return B200P_E_LENGTH;
-        return b200p_fa_rows_f32(step == 0 ? 0 : 1, 64, static_cast<const float*>(Q), static_cast<const float*>(K),
-                                 static_cast<const float*>(V), static_cast<float*>(O), batch, heads, seq_q, D, scale, stream);
+        if ((long long)batch * heads > 65535) return B200P_E_RANGE;
+        m_first = -3.402823466e+38f;
+        if (step == 2) step = 1;                           // the reference has no asynchronous form of those
     }
     switch (dtype) {
-        case B200P_F16:  return launch_step_d<__half>(step, D, Q, K, V, O, batch, heads, seq_q, seq_k, scale, st);
-        case B200P_BF16: return launch_step_d<__nv_bfloat16>(step, D, Q, K, V, O, batch, heads, seq_q, seq_k, scale, st);
-        default:         return launch_step_d<float>(step, D, Q, K, V, O, batch, heads, seq_q, seq_k, scale, st);
+        case B200P_F16:  return launch_step_d<__half>(step, D, Q, K, V, O, batch, heads, seq_q, seq_k, scale, m_first, st);
+        case B200P_BF16: return launch_step_d<__nv_bfloat16>(step, D, Q, K, V, O, batch, heads, seq_q, seq_k, scale, m_first, st);
+        default:         return launch_step_d<float>(step, D, Q, K, V, O, batch, heads, seq_q, seq_k, scale, m_first, st);
     }
 }

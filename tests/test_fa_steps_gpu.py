@@ -113,7 +113,7 @@ def test_fp32_row_kernels_ragged_and_wide_tiles(b200p, torch_cuda, variant, bc, 
 
 @pytest.mark.parametrize("step", STEPS[:3])
 def test_fp32_steps_accept_ragged_lengths(b200p, torch_cuda, step):
-    """b200p_fa_step with fp32 I/O and a length off the Br = 16 / Bc = 64 tiling takes the row kernels."""
+    """b200p_fa_step with fp32 I/O and a length off the Br = 16 / Bc = 64 tiling: padded keys and rows."""
     torch = torch_cuda
     D, S, H = 64, 203, 4
     rng = np.random.default_rng(0xB201)
@@ -137,3 +137,22 @@ def test_argument_errors(b200p, torch_cuda):
     with pytest.raises(b200p.B200PError) as e:
         b200p.fa_step("mfma2", Q, Q, Q)                     # the tensor-core step takes 16-bit operands
     assert e.value.status == -2
+
+
+# one key, the edges of a warp's 2 rows, of the 16 rows of a CTA and of the 64 keys of a tile, several tiles
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("S", [1, 2, 3, 15, 17, 63, 64, 65, 127, 130, 333])
+def test_fp32_steps_at_tile_edges(b200p, torch_cuda, S, D):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v = (torch.randn((2, 3, S, D), device="cuda", generator=g) for _ in range(3))
+    ref = (q.double() @ k.double().transpose(-1, -2) * D ** -0.5).softmax(-1) @ v.double()
+    outs = [b200p.fa_step(s, q, k, v) for s in STEPS[:3]]
+    for o in outs:
+        # scores of size 10 with 128 products each: relative error of a weight below 1e-5, values below 5
+        assert (o.double() - ref).abs().max() < 1e-4
+    assert torch.equal(outs[1], outs[2])
+    # scores below the running max's usual start: lengths off the tiling start at the lowest float
+    if S % 64:
+        q2 = torch.ones_like(q); k2 = torch.full_like(k, -2e38 / D)
+        assert (b200p.fa_step("dpp", q2, k2, v, scale=1.0).double() - v.double().mean(2, keepdim=True)).abs().max() < 1e-4

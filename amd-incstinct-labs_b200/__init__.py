@@ -156,15 +156,27 @@ def set_tuning(key: str, value: int) -> int:
     return int(lib().b200p_set_tuning(key.encode(), int(value)))
 
 
+_CODES = {}
+
+
 def _dtype_code(t) -> int:
-    import torch
-    return {torch.float32: F32, torch.float64: F64, torch.int32: I32, torch.int64: I64,
-            torch.float16: F16, torch.bfloat16: BF16}[t.dtype]
+    if not _CODES:
+        import torch
+        _CODES.update({torch.float32: F32, torch.float64: F64, torch.int32: I32, torch.int64: I64, torch.float16: F16, torch.bfloat16: BF16})
+    return _CODES[t.dtype]
+
+
+_raw_stream = None
 
 
 def _stream(t) -> int:
-    import torch
-    return torch.cuda.current_stream(t.device).cuda_stream
+    """The current stream of the tensor's device, asked for on every call.  The handle itself: a Stream object around it costs
+    more than the rest of a small call's arguments."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda i: torch.cuda.current_stream(i).cuda_stream)
+    return _raw_stream(t.get_device())
 
 
 def _dev(t, name: str):
@@ -189,7 +201,7 @@ def segreduce(x, op: str = "sum", out=None, narrow: bool = False):
     else:
         out_dtype = torch.float32 if code in (F16, BF16) else x.dtype
     if out is None:
-        out = torch.empty(nseg, dtype=out_dtype, device=x.device)
+        out = x.new_empty(nseg, dtype=out_dtype)
     fn = lib().b200p_segreduce_narrow if narrow else lib().b200p_segreduce
     _check(fn(OPS[op], code, x.data_ptr(), out.data_ptr(), x.numel(), _stream(x)), "segreduce")
     return out

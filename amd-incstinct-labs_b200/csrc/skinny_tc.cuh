@@ -13,10 +13,17 @@
 //    allows, from before the dependency wait on; one thread issues tcgen05.mma with W as A (M = 128) and X as B
 //    (N = 8 or 16), so no register and no warp touches the weights.  (An MMA takes about 40 cycles for any N up to 64,
 //    with 64 rows of W as with 128: tiles of 64 rows made the issue of the MMAs slower than HBM.);
+//  * two MMAs (32 columns of K) share an accumulator; the workers add the accumulators in fp32 registers, rounded to
+//    nearest.  An MMA that accumulates truncates: n of them in a row are off by about 2e-8 n on products of one sign, all
+//    downwards, and one accumulator for a whole slice made the outputs up to 25 times less exact than skinny_gemm.cuh's
+//    kernels, whose chains are K / 512 long (relative error over normal inputs, 16 rows: N = 32000, K = 2048 9.4e-8 with those
+//    kernels, 2.1e-6 with one accumulator a slice, 9.5e-8 now; 4096 x 4096 4.7e-7, 1.0e-6, 8.7e-8; 2048 x 5632 6.6e-7, 9.1e-7,
+//    9.2e-8).  One MMA per accumulator is 3 % closer still and 4 to 12 % slower (the workers then read as many bytes of
+//    tensor memory as the MMAs read of W: head of 32000 x 4096, 16 rows, 60.2 against 53.9 us; 51.7 with one accumulator a slice);
 //  * the partial accumulators are pushed to the CTA of the cluster that owns the outputs (64 / CS row pairs each),
 //    again with st.async; the owner adds the CS parts in slice order (the result does not depend on timing) and runs
-//    the epilogue.  Accumulators in tensor memory and the inboxes are double-buffered: the products of the next tile
-//    run under the exchange of this one.
+//    the epilogue.  Accumulators in tensor memory are a ring of kStcSlots blocks and the inboxes are double-buffered: the
+//    products of the next tile begin under the exchange of this one.
 // What bounds it: the stream of W (HBM), and for one or two tiles per cluster the chain dependency wait -> X -> last
 // stage's products -> exchange -> epilogue.  The shared memory is kept below half an SM's where the ring allows, so that the
 // next kernel's CTAs are resident and fetch their first stages under this one (the decode step: 15.6 -> 14.8 ms).
@@ -42,6 +49,14 @@ constexpr int kStcWorkers = 256;
 constexpr int kStcThreads = kStcWorkers + 64;             // + producer warp + MMA warp
 constexpr int kStcMaxStages = 12;
 constexpr int kStcMaxCluster = 8;
+constexpr int kStcAccs = 2;                               // accumulators of a block, 16 columns of tensor memory apart
+constexpr int kStcSlots = 8;                              // blocks between the MMA warp and the workers
+constexpr int kStcSlotCols = kStcAccs * 16;
+constexpr int kStcTmemCols = kStcSlots * kStcSlotCols;
+// At least a third of an SM's shared memory, so that no more CTAs meet on an SM than its tensor memory serves: a CTA that waited
+// for tensor memory could hold up its cluster, and that cluster another one.
+constexpr int kStcMinDynamic = 78 * 1024;
+static_assert(2 * kStcTmemCols <= 512 && 3 * (kStcMinDynamic + 1024) > 228 * 1024, "two CTAs on an SM, not three");
 
 struct SkinnyTcShape {
     int cluster;          // CTAs sharing K
@@ -287,7 +302,7 @@ skinny_tc_kernel(const SkinnyArgs a, const SkinnyTcShape sh, const __grid_consta
     griddep_launch_dependents();
     extern __shared__ __align__(1024) unsigned char stc_raw[];
     unsigned char* const stc_smem = stc_raw + (-dme::smem_addr(stc_raw) & 1023u);      // swizzle atoms start on 1 KB, wherever the linker put the array
-    __shared__ uint64_t full[kStcMaxStages], empty[kStcMaxStages], acc_full[2], acc_empty[2], inbox_full[2], x_full, ss_full, drained;
+    __shared__ uint64_t full[kStcMaxStages], empty[kStcMaxStages], prod_full[kStcSlots], prod_empty[kStcSlots], inbox_full[2], x_full, ss_full, drained;
     __shared__ float ss[16 * kStcMaxCluster];
     __shared__ uint32_t s_tmem;
     constexpr int ROW = stc_inbox_row(NB);
@@ -303,13 +318,14 @@ skinny_tc_kernel(const SkinnyArgs a, const SkinnyTcShape sh, const __grid_consta
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < sh.nstages; ++s) { dme::mbar_init(&full[s], 1); dme::mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { dme::mbar_init(&acc_full[b], 1); dme::mbar_init(&acc_empty[b], kStcWorkers / 32); dme::mbar_init(&inbox_full[b], 1); }
+        for (int b = 0; b < kStcSlots; ++b) { dme::mbar_init(&prod_full[b], 1); dme::mbar_init(&prod_empty[b], kStcWorkers / 32); }
+        for (int b = 0; b < 2; ++b) dme::mbar_init(&inbox_full[b], 1);
         dme::mbar_init(&x_full, PRO == PRO_PLAIN ? 1 : kStcWorkers);
         dme::mbar_init(&ss_full, 1);
         dme::mbar_init(&drained, 1);
         dme::mbar_init_fence();
     }
-    if (warp == kStcWorkers / 32 + 1) { tc::tmem_alloc(&s_tmem, 32); tc::tmem_relinquish(); }
+    if (warp == kStcWorkers / 32 + 1) { tc::tmem_alloc(&s_tmem, kStcTmemCols); tc::tmem_relinquish(); }
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -365,30 +381,34 @@ skinny_tc_kernel(const SkinnyArgs a, const SkinnyTcShape sh, const __grid_consta
     } else if (warp == kStcWorkers / 32 + 1) {
         // ---- MMA issuer: all lanes walk the loop, one issues (tc::elect_one) --------------------------------------
         constexpr uint32_t idesc = tc::instr_desc_f16(kStcRows, NB, StcFmt<T>::id, 0, 0);
-        int stage = 0; uint32_t phase = 0;
-        int it = 0;
+        int stage = 0, use = 0; uint32_t phase = 0;
         auto wait = [&](uint64_t* bar, uint32_t parity) { ok = __all_sync(0xffffffffu, dme::wait(bar, parity, status)) != 0; return ok; };
         const uint64_t a0 = tc::smem_desc_sw128(dme::smem_addr(stages), 16, 1024), b0 = tc::smem_desc_sw128(dme::smem_addr(xs), 16, 1024);
         wait(&x_full, 0);
-        bool ready = false;                                       // the stage's bytes were seen to be there, asked ahead of the MMAs before it:
-        for (int tile = cluster; tile < sh.ntiles && ok; tile += nclusters, ++it) {       // a wait takes 130 cycles even when there is nothing to wait for
-            const int b = it & 1;
-            if (it >= 2 && !wait(&acc_empty[b], uint32_t(((it >> 1) - 1) & 1))) break;
+        // the blocks take the slots in turn; what was in a slot before must have been read
+        auto slot_parity = [](int u) { return uint32_t(u / kStcSlots - 1) & 1u; };
+        bool bytes = false, room = true;                          // seen to be there, asked ahead of the MMAs before:
+        for (int tile = cluster; tile < sh.ntiles && ok; tile += nclusters) {             // a wait takes 130 cycles even when there is nothing to wait for
             for (int k = 0; k < nblk; ++k) {
-                if (!ready && !wait(&full[stage], phase)) break;
+                const int slot = use % kStcSlots;
+                if (!bytes && !wait(&full[stage], phase)) break;
+                if (!room && !wait(&prod_empty[slot], slot_parity(use))) break;
                 tc::fence_after_sync();
                 const uint64_t ad = a0 + uint64_t(stage * (kStcStageBytes / 16)), bd = b0 + uint64_t(k * (NB * 128 / 16));
                 uint64_t* const freed = &empty[stage];
+                ++use;
                 if (++stage == sh.nstages) { stage = 0; phase ^= 1u; }
-                const bool next = dme::mbar_test_wait(&full[stage], phase);
+                const bool next_bytes = dme::mbar_test_wait(&full[stage], phase);
+                const bool next_room = use < kStcSlots || dme::mbar_test_wait(&prod_empty[use % kStcSlots], slot_parity(use));
                 if (tc::elect_one()) {
                     #pragma unroll
                     for (int s = 0; s < 4; ++s)
-                        tc::mma_ss(tmem + b * 16, ad + uint64_t(s * 2), bd + uint64_t(s * 2), idesc, (k | s) != 0);
+                        tc::mma_ss(tmem + slot * kStcSlotCols + s * kStcAccs / 4 * 16, ad + uint64_t(s * 2), bd + uint64_t(s * 2), idesc, s * kStcAccs % 4 != 0);
                     tc::commit(freed);
-                    if (k == nblk - 1) tc::commit(&acc_full[b]);
+                    tc::commit(&prod_full[slot]);
                 }
-                ready = __all_sync(0xffffffffu, next) != 0;
+                bytes = __all_sync(0xffffffffu, next_bytes) != 0;
+                room = __all_sync(0xffffffffu, next_room) != 0;
             }
         }
         if (!ok) {                                                // the products in flight end before tensor memory is freed
@@ -415,10 +435,11 @@ skinny_tc_kernel(const SkinnyArgs a, const SkinnyTcShape sh, const __grid_consta
             dme::fence_proxy_async_smem();
             dme::mbar_arrive(&x_full);
         }
+        constexpr int HB = NB / 2;
         const int quarter = warp % 4, h = warp / 4;               // TMEM lanes of the warp; half of the NB columns
         const int2 pr = stc_pair<EPI>(a, 32 * quarter + lane);
-        const int owner = pr.x / per, slot = (pr.x % per) * 2 + pr.y;
-        int it = 0;
+        const int owner = pr.x / per, row = (pr.x % per) * 2 + pr.y;
+        int it = 0, use = 0;
         for (int tile = cluster; tile < sh.ntiles; tile += nclusters, ++it) {
             const int b = it & 1;
             float* box = inbox + b * inbox_floats;
@@ -429,17 +450,33 @@ skinny_tc_kernel(const SkinnyArgs a, const SkinnyTcShape sh, const __grid_consta
                 const int idx = tid + u * kStcWorkers;
                 if (idx < mine * NB) ahead[u] = stc_fetch<T, EPI>(a, tile, rank * per + idx % mine, idx / mine);
             }
-            if (ok && !dme::wait(&acc_full[b], uint32_t((it >> 1) & 1), status)) ok = false;
-            __syncwarp();
-            tc::fence_after_sync();
-            uint32_t v[8];
-            tc::ld_32x32b<NB / 2>(tc::tmem_addr(tmem, 32 * quarter, b * 16 + h * (NB / 2)), v);
-            tc::wait_ld();
-            tc::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) dme::mbar_arrive(&acc_empty[b]);
+            // the blocks' products, in two sums that take turns
+            float sum[HB], other[HB];
+            #pragma unroll
+            for (int j = 0; j < HB; ++j) sum[j] = other[j] = 0.f;
+            for (int k = 0; k < nblk; ++k, ++use) {
+                const int slot = use % kStcSlots;
+                if (ok && !dme::wait(&prod_full[slot], uint32_t(use / kStcSlots) & 1u, status)) ok = false;
+                __syncwarp();
+                tc::fence_after_sync();
+                uint32_t v[kStcAccs][HB];
+                #pragma unroll
+                for (int s = 0; s < kStcAccs; ++s) tc::ld_32x32b<HB>(tc::tmem_addr(tmem, 32 * quarter, slot * kStcSlotCols + s * 16 + h * HB), v[s]);
+                tc::wait_ld();
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) dme::mbar_arrive(&prod_empty[slot]);
+                #pragma unroll
+                for (int j = 0; j < HB; ++j) {
+                    const float next = sum[j] + (__uint_as_float(v[0][j]) + __uint_as_float(v[1][j]));
+                    sum[j] = other[j]; other[j] = next;
+                }
+            }
+            uint32_t v[HB];
+            #pragma unroll
+            for (int j = 0; j < HB; ++j) v[j] = __float_as_uint(sum[j] + other[j]);
             {
-                const uint32_t dst = cluster_addr(dme::smem_addr(box + (size_t(rank) * 2 * per + slot) * ROW + h * (NB / 2)), uint32_t(owner));
+                const uint32_t dst = cluster_addr(dme::smem_addr(box + (size_t(rank) * 2 * per + row) * ROW + h * HB), uint32_t(owner));
                 const uint32_t bar = cluster_addr(dme::smem_addr(&inbox_full[b]), uint32_t(owner));
                 #pragma unroll
                 for (int j = 0; j < NB / 8; ++j) st_async_v4(dst + 16 * j, v + 4 * j, bar);
@@ -468,7 +505,7 @@ skinny_tc_kernel(const SkinnyArgs a, const SkinnyTcShape sh, const __grid_consta
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     tc::fence_after_sync();
-    if (warp == kStcWorkers / 32 + 1) tc::tmem_dealloc(tmem, 32);
+    if (warp == kStcWorkers / 32 + 1) tc::tmem_dealloc(tmem, kStcTmemCols);
 }
 
 // Whether the shape is in the domain of this kernel and the other two: K a multiple of 16 (32-byte steps along the rows of W
@@ -558,7 +595,8 @@ int launch_skinny_tc(const SkinnyArgs& a, cudaStream_t st) {
         if (int se = take_launch_slot(st, &slot)) return se;
         status = slot.abort;
     }
-    const size_t dyn = 1024 + size_t(sh.x_bytes) + size_t(sh.nstages) * kStcStageBytes + size_t(boxes) * sh.inbox_bytes;
+    size_t dyn = 1024 + size_t(sh.x_bytes) + size_t(sh.nstages) * kStcStageBytes + size_t(boxes) * sh.inbox_bytes;
+    if (dyn < size_t(kStcMinDynamic)) dyn = size_t(kStcMinDynamic);
     auto kern = skinny_tc_kernel<T, PRO, EPI, NB>;
     if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn))) return int(e);
     return launch_dependent_clusters(kern, best, dim3(unsigned(clusters * best)), kStcThreads, dyn, st, a, sh, mw, mx, status, sticky);

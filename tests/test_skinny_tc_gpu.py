@@ -64,3 +64,16 @@ def test_gated_epilogues(b200p, torch_cuda, M, F, K):
     ref = g / (1.0 + np.exp(-g)) * u
     b200p.skinny_gemm(W, out, x32=torch.from_numpy(x).cuda(), norm_w=nw, epilogue="silu16")
     assert np.abs(out.float().cpu().numpy() - ref).max() < (2.0 ** -8 + 3e-3) * max(1e-3, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 300, 8192), (16, 300, 4096), (16, 520, 2048), (11, 200, 1040)])
+def test_products_of_one_sign_are_not_truncated_in_long_chains(b200p, torch_cuda, cluster, M, N, K):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(K)
+    W, X = (torch.randn(s, device="cuda", generator=g).abs().bfloat16() for s in ((N, K), (M, K)))
+    out = torch.zeros((M, N), device="cuda")
+    b200p.skinny_gemm(W, out, x16=X, epilogue="acc32")
+    ref = X.double() @ W.double().T
+    # two truncated additions lose at most 2^-23 of the sum each; the fp32 sums after them round to nearest, which averages
+    # out, below 2^-24.  One accumulator for all of K = 4096: 256 truncations, 5e-6.
+    assert ((out.double() - ref).norm() / ref.norm()).item() < 2 * 2.0 ** -23 + 2.0 ** -24

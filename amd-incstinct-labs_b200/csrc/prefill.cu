@@ -17,21 +17,21 @@ struct PrefillPlan {
 // The heads of a group share their keys, and where their rows follow one another in memory they can be one run of
 // group * seqQ rows: fewer items at ragged lengths, and the last item of a head is not mostly padding.  Taken where it saves a
 // round of items over the SMs (fp16, 32 / 4 heads of 64, 2 x 1111 tokens: 320 items are three rounds, 280 are two: 53.5 -> 41.0
-// us; causal 2 x 555: 192 -> 144 items, 21.4 -> 18.6 us).  Causal tiles that run over a head's end see all keys, which costs more than
-// it saves when the rounds stay the same (64 / 8 heads, 700 tokens, 192 -> 176 items: 24.8 -> 28.8 us; 2500: 112 -> 126 us), so there
-// only down to at most two rounds.
+// us).  Under the causal mask only where no tile runs over a head's end.  Such a tile has to see the keys of its last row, and
+// the rows after the head's end would multiply values behind their own position by zero: a NaN or infinity there reached rows
+// that may not see it.  (It also lost time where each tile then saw all keys: 8 x 8 / 1 heads of 64, 1111 tokens 39.0 -> 44.2 us.)
 // An item is two tiles because their softmax and products overlap; a tile alone takes 0.6 of a pair's time.  Where every
 // tile can have an SM of its own, single tiles are the faster form (1 head, 5000 keys, causal: 71.7 -> 58.1 us; 8 heads, 512 keys:
 // 14.4 -> 12.4), else pairs are (32 heads, 1024 tokens: 24.7 against 35.2); under four key tiles there is nothing to overlap.
 PrefillPlan prefill_plan(const b200p_prefill_cfg* c, const b200p_attn_strides& s) {
     const int v = tuning(KNOB_PREFILL_VARIANT, 0);
     const long long group = c->nQHeads / c->nKVHeads, sms = sm_count();
-    const bool can_pack = group > 1 && s.q_head == c->seqQ * s.q_seq && s.o_head == c->seqQ * s.o_seq && c->seqQ * group < (1 << 30);
+    const bool can_pack = group > 1 && (!c->causal || c->seqQ % kBM == 0) && s.q_head == c->seqQ * s.q_seq && s.o_head == c->seqQ * s.o_seq && c->seqQ * group < (1 << 30);
     if (v & 16) return {v & 4 ? 1 : 2, (v & 8) != 0 && can_pack};
     auto items = [&](long long rows, long long heads, int span) { return (rows + span * kBM - 1) / (span * kBM) * heads * c->batch; };
     auto rounds = [&](long long n) { return (n + sms - 1) / sms; };
     const long long alone = rounds(items(c->seqQ, c->nQHeads, 2)), together = rounds(items(c->seqQ * group, c->nKVHeads, 2));
-    PrefillPlan p{2, can_pack && together < alone && (!c->causal || together <= 2)};
+    PrefillPlan p{2, can_pack && together < alone};
     const long long tiles = p.packed ? items(c->seqQ * group, c->nKVHeads, 1) : items(c->seqQ, c->nQHeads, 1);
     if (tiles <= sms && c->seqK > 3 * kBN) p.span = 1;
     return p;
@@ -76,7 +76,7 @@ int launch_prefill_rs(const void* Q, const void* K, const void* V, void* O, cons
     if (int se = take_launch_slot(st, &slot)) return se;       // work counter and abort word of this launch, cleared on its stream
     p.status = slot.abort; p.work_counter = slot.work;
     p.seqQ = c->seqQ * per; p.seqK = c->seqK; p.nQH = heads; p.nKVH = c->nKVHeads; p.group = plan.packed ? 1 : group;
-    p.span = plan.span; p.pack = plan.packed ? c->seqQ : 0;
+    p.span = plan.span; p.pack = plan.packed && c->causal ? c->seqQ : 0;
     p.batch = c->batch; p.causal = c->causal;
     p.scale_log2 = 1.4426950408889634f / sqrtf(float(D));
     // One persistent CTA per SM (the kernel takes all of an SM's shared and tensor memory), or one CTA per

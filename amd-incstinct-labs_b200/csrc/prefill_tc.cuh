@@ -101,7 +101,7 @@ struct PrefillParams {
     int seqQ, seqK, nQH, nKVH, group, batch, causal;
     float scale_log2;
     int span;                  // query tiles per item: 2, or 1 where pairs would leave SMs idle
-    int pack;                  // the query heads of a group are one run of rows: a row's position is row % pack (0: each head on its own)
+    int pack;                  // causal, the query heads of a group as one run of rows, whole tiles each: a row's position is row % pack (0: the row)
     // PORTION shapes only
     int pos0;                  // keys cached before the first query row: row i sees keys <= pos0 + i
     int v_cols;                // value columns that exist
@@ -137,10 +137,7 @@ __device__ __forceinline__ PrefillItem prefill_item(const PrefillParams& p, int 
     for (int t = 0; t < 2; ++t) {
         w.q0[t] = qb * rows + t * kBM;
         if (w.q0[t] >= p.seqQ || t >= p.span) w.n[t] = 0;
-        else if (!Sh::PORTION && p.causal && p.pack) {
-            const int last = w.q0[t] % p.pack + min(kBM, p.seqQ - w.q0[t]) - 1;
-            w.n[t] = min(ntk, min(last, p.pack - 1) / kBN + 1);
-        }
+        else if (!Sh::PORTION && p.pack) w.n[t] = min(ntk, (w.q0[t] % p.pack + kBM - 1) / kBN + 1);
         else if (p.causal) w.n[t] = min(ntk, ((Sh::PORTION ? p.pos0 : 0) + w.q0[t] + kBM - 1) / kBN + 1) - w.first;
         else w.n[t] = ntk - w.first;
     }
@@ -404,11 +401,7 @@ prefill_tc_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap map
           const int o_b = w.b, o_head = w.head;
           const int row = q0t + r;
           int row_pos = PORTION ? p.pos0 + row : row, q0_pos = PORTION ? p.pos0 + q0t : q0t;      // of the row, least of the tile
-          if (!PORTION && p.pack) {
-              row_pos = row % p.pack;
-              q0_pos = q0t % p.pack;
-              if (q0_pos + kBM > p.pack) q0_pos = 0;
-          }
+          if (!PORTION && p.pack) { q0_pos = q0t % p.pack; row_pos = q0_pos + r; }
           const int first_key = MASKED ? p.mask.first(row_pos) : 0, last_first = MASKED ? p.mask.first(q0_pos + kBM - 1) : 0;
           float m_used = -INFINITY, l = 0.f;
           if (MASKED) { m_used = p.plus_one ? 0.f : -1e30f; l = p.plus_one ? 1.f : 0.f; }      // finite: a row may see nothing of its first tiles

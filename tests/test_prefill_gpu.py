@@ -191,3 +191,16 @@ def test_work_items_of_every_form_give_the_same_bits(b200p, torch_cuda, D, causa
     if causal:
         s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
     assert (outs[0].double() - s.softmax(-1) @ vd).abs().max() < 2e-2
+
+
+# lengths whose last tile is not full, groups, sizes at which the heads of a group would fit fewer rounds of items as one run of rows
+@pytest.mark.parametrize("batch,heads,kv,S,D", [(2, 32, 4, 555, 64), (2, 32, 8, 1111, 128), (8, 8, 1, 1111, 64), (8, 64, 8, 128, 64), (8, 64, 8, 384, 64), (1, 8, 8, 300, 64)])
+def test_values_behind_a_rows_position_do_not_reach_it(b200p, torch_cuda, batch, heads, kv, S, D):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v = (torch.randn((batch, h, S, D), device="cuda", generator=g).bfloat16() for h in (heads, kv, kv))
+    clean = b200p.prefill(q, k, v, causal=True)
+    for bad in (float("nan"), float("inf")):
+        v2 = v.clone(); v2[:, :, S - 3:] = bad
+        first = (S - 3) // 128 * 128                                 # rows that share a tile of keys with the bad ones may see 0 x bad
+        assert torch.equal(b200p.prefill(q, k, v2, causal=True)[:, :, :first], clean[:, :, :first])

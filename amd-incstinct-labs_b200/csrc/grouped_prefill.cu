@@ -34,13 +34,14 @@ int launch(const GroupedAttn& a, cudaStream_t st) {
     PrefillParams p{};
     p.sticky = device_status_ptr();
     if (!p.sticky) return B200P_E_NO_DEVICE;
-    const long long items = (long long)((a.Tn + 2 * kBM - 1) / (2 * kBM)) * d.heads * a.batch;
+    const int blocks = (a.Tn + 2 * kBM - 1) / (2 * kBM);
+    const long long items = (long long)blocks * d.heads * a.batch;
     if (items > 0x7fffffffLL / 2) return B200P_E_RANGE;
     LaunchSlot slot{};
     if (int se = take_launch_slot(st, &slot)) return se;
     p.status = slot.abort; p.work_counter = slot.work;
     p.seqQ = a.Tn; p.seqK = N; p.nQH = d.heads; p.nKVH = d.kv_heads; p.group = d.group(); p.batch = a.batch; p.causal = 1;
-    p.scale_log2 = a.scale * 1.4426950408889634f; p.span = 2;
+    p.scale_log2 = a.scale * 1.4426950408889634f; p.span = 2; p.blocks = blocks; p.items = int(items);
     p.pos0 = a.pos0; p.v_cols = d.vdim; p.mask = a.mask; p.plus_one = a.plus_one ? 1 : 0;
     const int sms = sm_count();
     kern<<<unsigned(items < sms ? items : sms), prefill_threads(1), Sh::SMEM_BYTES, st>>>(p, mq, mk, mv, mo, mq, mk);

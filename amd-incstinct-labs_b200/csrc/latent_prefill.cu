@@ -41,10 +41,12 @@ int launch(const LatentAttn& a, cudaStream_t st) {
     if (int se = take_launch_slot(st, &slot)) return se;
     p.status = slot.abort; p.work_counter = slot.work;
     p.seqQ = a.Tn; p.seqK = N; p.nQH = p.nKVH = d.heads; p.group = 1; p.batch = a.batch; p.causal = 1;
-    p.scale_log2 = a.scale * 1.4426950408889634f; p.span = 2;
+    p.scale_log2 = a.scale * 1.4426950408889634f;
     p.pos0 = a.pos0; p.v_cols = d.vdim; p.sink = a.sink;
-    const long long items = (long long)((a.Tn + 2 * kBM - 1) / (2 * kBM)) * d.heads * a.batch;
+    p.span = 2; p.blocks = (a.Tn + 2 * kBM - 1) / (2 * kBM);
+    const long long items = (long long)p.blocks * d.heads * a.batch;
     if (items > 0x7fffffffLL / 2) return B200P_E_RANGE;
+    p.items = int(items);
     const int sms = sm_count();
     kern<<<unsigned(items < sms ? items : sms), prefill_threads(1), Sh::SMEM_BYTES, st>>>(p, mq, mk, mv, mo, mqr, mkr);
     if (int le = launched()) return le;

@@ -17,16 +17,17 @@ struct PrefillPlan {
 // The heads of a group share their keys, and where their rows follow one another in memory they can be one run of
 // group * seqQ rows: fewer items at ragged lengths, and the last item of a head is not mostly padding.  Taken where it saves a
 // round of items over the SMs (fp16, 32 / 4 heads of 64, 2 x 1111 tokens: 320 items are three rounds, 280 are two: 53.5 -> 41.0
-// us).  Under the causal mask only where no tile runs over a head's end.  Such a tile has to see the keys of its last row, and
-// the rows after the head's end would multiply values behind their own position by zero: a NaN or infinity there reached rows
-// that may not see it.  (It also lost time where each tile then saw all keys: 8 x 8 / 1 heads of 64, 1111 tokens 39.0 -> 44.2 us.)
+// us).  Not under the causal mask: a tile that runs over a head's end has to see the keys of its last row, and the rows after the
+// head's end would multiply values behind their own position by zero, so that a NaN or infinity there reached rows that may not
+// see it.  (It also lost time where each tile then saw all keys: 8 x 8 / 1 heads of 64, 1111 tokens 39.0 -> 44.2 us; and rows that wrap
+// to a position cost every item a division.)
 // An item is two tiles because their softmax and products overlap; a tile alone takes 0.6 of a pair's time.  Where every
 // tile can have an SM of its own, single tiles are the faster form (1 head, 5000 keys, causal: 71.7 -> 58.1 us; 8 heads, 512 keys:
 // 14.4 -> 12.4), else pairs are (32 heads, 1024 tokens: 24.7 against 35.2); under four key tiles there is nothing to overlap.
 PrefillPlan prefill_plan(const b200p_prefill_cfg* c, const b200p_attn_strides& s) {
     const int v = tuning(KNOB_PREFILL_VARIANT, 0);
     const long long group = c->nQHeads / c->nKVHeads, sms = sm_count();
-    const bool can_pack = group > 1 && (!c->causal || c->seqQ % kBM == 0) && s.q_head == c->seqQ * s.q_seq && s.o_head == c->seqQ * s.o_seq && c->seqQ * group < (1 << 30);
+    const bool can_pack = group > 1 && !c->causal && s.q_head == c->seqQ * s.q_seq && s.o_head == c->seqQ * s.o_seq && c->seqQ * group < (1 << 30);
     if (v & 16) return {v & 4 ? 1 : 2, (v & 8) != 0 && can_pack};
     auto items = [&](long long rows, long long heads, int span) { return (rows + span * kBM - 1) / (span * kBM) * heads * c->batch; };
     auto rounds = [&](long long n) { return (n + sms - 1) / sms; };
@@ -76,13 +77,15 @@ int launch_prefill_rs(const void* Q, const void* K, const void* V, void* O, cons
     if (int se = take_launch_slot(st, &slot)) return se;       // work counter and abort word of this launch, cleared on its stream
     p.status = slot.abort; p.work_counter = slot.work;
     p.seqQ = c->seqQ * per; p.seqK = c->seqK; p.nQH = heads; p.nKVH = c->nKVHeads; p.group = plan.packed ? 1 : group;
-    p.span = plan.span; p.pack = plan.packed && c->causal ? c->seqQ : 0;
+    p.span = plan.span;
     p.batch = c->batch; p.causal = c->causal;
     p.scale_log2 = 1.4426950408889634f / sqrtf(float(D));
     // One persistent CTA per SM (the kernel takes all of an SM's shared and tensor memory), or one CTA per
     // work item when the knob's bit 1 is set.
-    const long long items = (long long)((p.seqQ + p.span * kBM - 1) / (p.span * kBM)) * heads * c->batch;
+    p.blocks = (p.seqQ + p.span * kBM - 1) / (p.span * kBM);
+    const long long items = (long long)p.blocks * heads * c->batch;
     if (items > 0x7fffffffLL / 2) return B200P_E_RANGE;
+    p.items = int(items);
     const int sms = sm_count();
     const bool one_per_item = (tuning(KNOB_PREFILL_VARIANT, 0) & 2) != 0;
     dim3 grid(unsigned(one_per_item || items < sms ? items : sms), 1, 1);

@@ -100,8 +100,8 @@ struct PrefillParams {
     int* work_counter;         // zero at launch: the CTAs draw the ids of their later work items from it
     int seqQ, seqK, nQH, nKVH, group, batch, causal;
     float scale_log2;
-    int span;                  // query tiles per item: 2, or 1 where pairs would leave SMs idle
-    int pack;                  // causal, the query heads of a group as one run of rows, whole tiles each: a row's position is row % pack (0: the row)
+    int span;                  // query tiles per item: 2, or 1 where pairs would leave SMs idle (PORTION shapes: 2)
+    int blocks, items;         // items of a head, of the launch; the host's divisions (in every role they cost a small call 0.5 us)
     // PORTION shapes only
     int pos0;                  // keys cached before the first query row: row i sees keys <= pos0 + i
     int v_cols;                // value columns that exist
@@ -126,18 +126,17 @@ struct PrefillItem {
 template <typename Sh>
 __device__ __forceinline__ PrefillItem prefill_item(const PrefillParams& p, int id) {
     PrefillItem w;
-    const int rows = p.span * kBM, nqb = (p.seqQ + rows - 1) / rows;
-    const int qb = nqb - 1 - id % nqb;
-    w.head = (id / nqb) % p.nQH;
-    w.b = id / (nqb * p.nQH);
+    const int span = Sh::PORTION ? 2 : p.span, rows = span * kBM;
+    const int bh = id / p.blocks, qb = p.blocks - 1 - (id - bh * p.blocks);
+    w.b = bh / p.nQH;
+    w.head = bh - w.b * p.nQH;
     w.kvh = w.head / p.group;
     const int ntk = (p.seqK + kBN - 1) / kBN;
     w.first = Sh::MASKED ? p.mask.first(p.pos0 + qb * rows) / kBN : 0;
     #pragma unroll
     for (int t = 0; t < 2; ++t) {
         w.q0[t] = qb * rows + t * kBM;
-        if (w.q0[t] >= p.seqQ || t >= p.span) w.n[t] = 0;
-        else if (!Sh::PORTION && p.pack) w.n[t] = min(ntk, (w.q0[t] % p.pack + kBM - 1) / kBN + 1);
+        if (w.q0[t] >= p.seqQ || t >= span) w.n[t] = 0;
         else if (p.causal) w.n[t] = min(ntk, ((Sh::PORTION ? p.pos0 : 0) + w.q0[t] + kBM - 1) / kBN + 1) - w.first;
         else w.n[t] = ntk - w.first;
     }
@@ -175,8 +174,6 @@ prefill_tc_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap map
     constexpr int kMmaWarp = 8 * RS, kTmaWarp = 8 * RS + 1;
     constexpr int kItemReaders = 2 * kBM + 1;                  // every softmax thread + the MMA thread
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int nqb = (p.seqQ + p.span * kBM - 1) / (p.span * kBM);
-    const int total_items = nqb * p.nQH * p.batch;
 
     if (threadIdx.x == 0) {
         s_failed = 0;
@@ -212,7 +209,8 @@ prefill_tc_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap map
     // Register budget: the softmax warpgroups hold a whole 128-column score row per thread, the MMA / TMA
     // warpgroup carries ring state, descriptors and the per-item bookkeeping; the three limits (multiples of 8) must
     // sum to no more than 3 x 168 = 504 (the launch allocation): 208 + 208 + 88.  Measured against 216 + 216 + 72:
-    // 16 instead of 44 bytes of spills in the D = 128 kernel (they sit in the 72-register branch), +3 % throughput.
+    // 16 instead of 44 bytes of spills in the D = 128 kernel of that time (they sit in the 72-register branch), +3 % throughput.
+    // Spills now, bytes stored / loaded: 16 / 40 at D = 128, 12 / 24 at 64, 28 / 40 masked, 236 / 324 in the widest latent form.
     // (Each role branch opens with its own setmaxnreg, so the compiler sees one limit per branch.)
     if (warp >= 8 * RS) {
       asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
@@ -227,7 +225,7 @@ prefill_tc_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap map
                 // draw and publish the item
                 if (it >= 2 && !dme::wait(&item_empty[it & 1], uint32_t(((it >> 1) - 1) & 1), p.status)) { ok = false; break; }
                 int id = it == 0 ? int(blockIdx.x) : int(gridDim.x) + atomicAdd(p.work_counter, 1);
-                if (id >= total_items) id = -1;
+                if (id >= p.items) id = -1;
                 s_item[it & 1] = id;
                 dme::mbar_arrive(&item_full[it & 1]);
                 if (id < 0) break;
@@ -400,8 +398,7 @@ prefill_tc_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap map
           const int q0t = t ? w.q0[1] : w.q0[0], nt = t ? w.n[1] : w.n[0];     // no arrays indexed at run time
           const int o_b = w.b, o_head = w.head;
           const int row = q0t + r;
-          int row_pos = PORTION ? p.pos0 + row : row, q0_pos = PORTION ? p.pos0 + q0t : q0t;      // of the row, least of the tile
-          if (!PORTION && p.pack) { q0_pos = q0t % p.pack; row_pos = q0_pos + r; }
+          const int row_pos = PORTION ? p.pos0 + row : row, q0_pos = PORTION ? p.pos0 + q0t : q0t;
           const int first_key = MASKED ? p.mask.first(row_pos) : 0, last_first = MASKED ? p.mask.first(q0_pos + kBM - 1) : 0;
           float m_used = -INFINITY, l = 0.f;
           if (MASKED) { m_used = p.plus_one ? 0.f : -1e30f; l = p.plus_one ? 1.f : 0.f; }      // finite: a row may see nothing of its first tiles

@@ -64,6 +64,11 @@ struct LaunchSlot { int* work; int* abort; };
 // B200P_OK, B200P_E_NO_DEVICE or the cudaError_t of the clearing memset.
 int take_launch_slot(cudaStream_t st, LaunchSlot* out);
 
+// Lets `kernel` be launched with `bytes` of dynamic shared memory.  The limit is state of the function on the device, which
+// all threads share: it is raised to all that the device allows on a kernel's first launch and never set to one launch's
+// size, which another thread's larger launch would then be refused for.  B200P_OK or the cudaError_t.
+int allow_dynamic_smem(const void* kernel, size_t bytes);
+
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 
 // Record a launch and translate the launch status.

@@ -3,6 +3,7 @@
 #include "common.cuh"
 #include <climits>
 #include <cstring>
+#include <map>
 #include <mutex>
 
 namespace b200p {
@@ -71,6 +72,25 @@ int take_launch_slot(cudaStream_t st, LaunchSlot* out) {
     if (cudaError_t e = cudaMemsetAsync(base, 0, 2 * sizeof(int), st)) return int(e);
     out->work = base; out->abort = base + 1;
     return B200P_OK;
+}
+
+int allow_dynamic_smem(const void* kernel, size_t bytes) {
+    static std::map<std::pair<const void*, int>, size_t> limits;        // as many entries as kernels
+    static std::mutex mu;
+    int dev = -1;
+    if (cudaError_t e = cudaGetDevice(&dev)) return int(e);
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& limit = limits[{kernel, dev}];
+    if (limit == 0) {
+        cudaFuncAttributes fa{};
+        int most = 0;
+        if (cudaError_t e = cudaFuncGetAttributes(&fa, kernel)) return int(e);
+        if (cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) return int(e);
+        const size_t room = size_t(most) - fa.sharedSizeBytes;
+        if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(room))) return int(e);
+        limit = room;
+    }
+    return bytes <= limit ? B200P_OK : int(cudaErrorInvalidValue);
 }
 
 unsigned tuning_epoch() { return g_tuning_epoch.load(std::memory_order_relaxed); }

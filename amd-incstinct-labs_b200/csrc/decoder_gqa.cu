@@ -280,7 +280,7 @@ bool mega_plan(const b200p_session* s, MegaPlan* out) {
         cudaGetLastError();
         return false;
     }
-    if (cudaFuncSetAttribute(pl.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(pl.dyn)) != cudaSuccess ||
+    if (allow_dynamic_smem(pl.kernel, pl.dyn) != B200P_OK ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pl.kernel, kSkinnyStreamThreads, pl.dyn) != cudaSuccess || per_sm < 1) {
         cudaGetLastError();
         return false;

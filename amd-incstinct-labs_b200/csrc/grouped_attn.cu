@@ -189,7 +189,7 @@ int launch_plain(const GroupedAttn& a, cudaStream_t st) {
     const size_t smem = (size_t(kPlainRows) * a.d.dim + size_t(kPlainKeys) * (a.d.dim + 1) + size_t(kPlainKeys) * a.d.vdim) * 4;
     auto kern = grouped_plain_kernel<T, NV>;
     if (smem > 48 * 1024)
-        if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) return int(e);
+        if (int e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) return e;
     kern<<<dim3(unsigned((a.Tn + kPlainRows - 1) / kPlainRows), unsigned(a.d.heads), unsigned(a.batch)), kPlainRows * 32, smem, st>>>(a);
     return launched();
 }

@@ -106,7 +106,7 @@ int launch_plain(const LatentAttn& a, cudaStream_t st) {
     if (smem > 220 * 1024) return B200P_E_DIM;
     auto kern = latent_plain_kernel<T, NV>;
     if (smem > 48 * 1024)
-        if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) return int(e);
+        if (int e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) return e;
     kern<<<dim3(unsigned((a.Tn + kPlainRows - 1) / kPlainRows), unsigned(a.d.heads), unsigned(a.batch)), kPlainRows * 32, smem, st>>>(a);
     return launched();
 }
@@ -600,7 +600,7 @@ int launch_attend(const LatentStep& a, const StepPlan& p, cudaStream_t st) {
     int* sticky = device_status_ptr();
     if (!sticky) return B200P_E_NO_DEVICE;
     auto kern = latent_attend_kernel<MT, NG>;
-    if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(p.smem))) return int(e);
+    if (int e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), p.smem)) return e;
     return launch_dependent(kern, dim3(unsigned(p.splits), unsigned(p.groups), unsigned(a.batch)), kStepThreads + 32, p.smem, st, a, map, p.splits, p.stages, sticky);
 }
 

@@ -830,8 +830,7 @@ int launch_skinny_mh(const SkinnyArgs& a, cudaStream_t st) {
             const int groups = groups_all;
             const size_t dyn = size_t(x_bytes) + size_t(nstages) * stage_bytes;
             void (*sk)(SkinnyArgs, int, int, int*, int*) = skinny_stream_kernel<T, PRO, EPI, MH>;
-            const cudaError_t ae = cudaFuncSetAttribute(sk, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn));
-            if (ae != cudaSuccess) return int(ae);
+            if (int e = allow_dynamic_smem(reinterpret_cast<const void*>(sk), dyn)) return e;
             cudaLaunchConfig_t cfg{};
             cfg.gridDim = dim3(groups < sms || one_group_ctas ? groups : sms); cfg.blockDim = dim3(kSkinnyStreamThreads); cfg.dynamicSmemBytes = dyn; cfg.stream = st;
             cudaLaunchAttribute attr[1];
@@ -851,8 +850,7 @@ int launch_skinny_mh(const SkinnyArgs& a, cudaStream_t st) {
     void (*kern)(SkinnyArgs) = skinny_gemm_kernel<T, PRO, EPI, 2, MH>;
     if constexpr (!paired) { if (half_rows) kern = skinny_gemm_kernel<T, PRO, EPI, 1, MH>; }
     if (smem > 28 * 1024) {                                     // static (8 or 16 KB) + dynamic beyond 48 KB needs the opt-in
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e != cudaSuccess) return int(e);
+        if (int e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) return e;
     }
     // Launched as a programmatic dependent: the CTAs may start while the previous kernel of the
     // stream is still draining, fetch their weights, and wait at griddep_wait() for its results.

@@ -603,7 +603,7 @@ int launch_skinny_tc(const SkinnyArgs& a, cudaStream_t st) {
     size_t dyn = 1024 + size_t(sh.x_bytes) + size_t(sh.nstages) * kStcStageBytes + size_t(boxes) * sh.inbox_bytes;
     if (dyn < size_t(kStcMinDynamic)) dyn = size_t(kStcMinDynamic);
     auto kern = skinny_tc_kernel<T, PRO, EPI, NB>;
-    if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn))) return int(e);
+    if (int e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), dyn)) return e;
     return launch_dependent_clusters(kern, best, dim3(unsigned(clusters * best)), kStcThreads, dyn, st, a, sh, mw, mx, status, sticky);
 }
 

@@ -41,7 +41,7 @@ enum Knob {
     KNOB_DELTA_PLAIN,           // 1: the gated delta rule token by token on the plain kernel
     KNOB_DELTA_COLUMNS,         // 1, 2 or 4: columns of S per lane (tensor-core form: 4, 2 or 1 warps per 16 columns) in the walk over blocks
     KNOB_DELTA_TENSOR,          // 0: blocks of 16-bit sessions without tensor cores as well
-    KNOB_SKINNY_CLUSTER,        // 1..8: CTAs that share K in skinny_tc_kernel (0: chosen from the shape)
+    KNOB_SKINNY_CLUSTER,        // 1..8: CTAs that share K in skinny_tc_kernel, where K has as many blocks of 64 columns (0: chosen from the shape)
     KNOB_COUNT
 };
 

@@ -24,7 +24,7 @@ int stc_resident_clusters(int cluster) {
     if (cudaFuncSetAttribute(stc_residency_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, stc_residency_kernel, &cfg) != cudaSuccess) {
         cudaGetLastError();
-        n = 0;
+        return 0;                                                   // asked again by the next call
     }
     kept.store(n + 1, std::memory_order_relaxed);
     return n;

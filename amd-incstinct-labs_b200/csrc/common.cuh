@@ -30,7 +30,7 @@ enum Knob {
     KNOB_RUNTIME_ROPE_FUSED,    // 1: RoPE + KV scatter in the Q/K/V projection's epilogue, 0: separate kernel
     KNOB_RUNTIME_SKINNY,        // decode-step projections: 0 library GEMMs, 1 skinny_gemm_kernel (W in registers),
                                 // 2 chosen from the shape (default): skinny_stream_kernel (W through shared memory) or
-                                // skinny_tc_kernel (K split over a cluster, tcgen05), 3 skinny_tc_kernel
+                                // skinny_tc_kernel (K split over a cluster, tcgen05), 3 skinny_tc_kernel or a range error
     KNOB_SCAN16_LANE,           // 1: 16-bit scans hold a whole segment per lane, 0: four lanes per segment
     KNOB_RUNTIME_GEMM,          // prefill projections: 1 the tcgen05 GEMM of this library (default), 0 library GEMMs
     KNOB_GEMM_TILE_N,           // 128 or 256: force the tensor-core GEMM's tile width (0: chosen from the shape)

@@ -619,7 +619,7 @@ int launch_skinny(const SkinnyArgs& a, cudaStream_t st) {
     const int kind = tuning(KNOB_RUNTIME_SKINNY, 2);
     if (kind == 3 || (kind == 2 && skinny_split(a.M, a.K, size_t(a.N) * a.K * (epi_gated(EPI) ? 4 : 2), a.abort_word != nullptr))) {
         const int e = a.M <= 8 ? launch_skinny_tc<T, PRO, EPI, 8>(a, st) : launch_skinny_tc<T, PRO, EPI, 16>(a, st);
-        if (e != B200P_E_RANGE) return e;
+        if (kind == 3 || e != B200P_E_RANGE) return e;
     }
     // up to 8 rows of X: one B fragment per A fragment; 9 .. 16 rows: two
     return a.M <= 8 ? launch_skinny_mh<T, PRO, EPI, 1>(a, st) : launch_skinny_mh<T, PRO, EPI, 2>(a, st);

@@ -1,9 +1,11 @@
-"""Decode steps of sessions on the projection kernel that splits K over a cluster, and what a session does where that kernel
-cannot run."""
+"""Decode steps of sessions on the projection kernel that splits K over a cluster: the forms that only sessions launch (rotated
+Q/K/V with the scatter into the cache, rotated query pairs, the prologue that adds the last sublayer's output), and what a
+session does where that kernel cannot run."""
 import numpy as np
 import pytest
 
 from oracle import runtime_ref as rr
+from test_latent_gpu import check, opened, reference, tokens  # noqa: F401 (opened is a fixture)
 from test_runtime_gpu import check_logits, to_device
 
 pytestmark = pytest.mark.gpu
@@ -38,3 +40,27 @@ def test_rows_too_long_for_every_allowed_split_take_the_gemm(b200p, torch_cuda):
     """8 rows of 12304 columns fit no streaming kernel, and one CTA of the cluster kernel neither."""
     b200p.set_tuning("skinny_cluster", 1)
     steps(b200p, torch_cuda, llama(4, 2, 64, ffn=12304, hidden=256), "bf16", False, 8)
+
+
+# heads whose rows fill the 128-row tiles and not, one head a tile and two, biases, one and two fragments of rows
+@pytest.mark.parametrize("cluster", [0, 1, 3, 8])
+@pytest.mark.parametrize("heads,kv,D,kind,bias,batch", [(8, 2, 64, "bf16", False, 1), (3, 3, 64, "f16", True, 3), (4, 1, 128, "bf16", True, 9), (5, 5, 64, "bf16", True, 16),
+                                                        (3, 1, 128, "f16", False, 16)])
+def test_rotated_projections(b200p, torch_cuda, cluster, heads, kv, D, kind, bias, batch):
+    b200p.set_tuning("runtime_skinny", 3)
+    b200p.set_tuning("skinny_cluster", cluster)
+    steps(b200p, torch_cuda, llama(heads, kv, D), kind, bias, batch)
+
+
+# 1 .. 4 rows form the residual sum in the next projection's prologue, more in a kernel of its own; then single tokens, which
+# read the cache that those rows wrote
+@pytest.mark.parametrize("cluster", [0, 1, 2, 8])
+@pytest.mark.parametrize("name", ["odd", "many_heads", "real_heads", "wide_mlp"])
+def test_latent_decoder(b200p, opened, name, cluster):  # noqa: F811
+    from test_latent_gpu import CONFIGS, run
+    b200p.set_tuning("runtime_skinny", 3)
+    b200p.set_tuning("skinny_cluster", cluster)
+    s, ids = opened(name, "bf16"), tokens(CONFIGS[name], 20, 2)
+    want = reference(name, ids)
+    for n in (1, 2, 3, 4, 5, 9, 16):
+        check(run(s, ids, [n, 1]), want, "bf16", n)

@@ -1,5 +1,6 @@
-"""The projection kernel that splits K over a cluster, forced for every shape and split: edges of its tiles (128 rows of W,
-64 pairs), of its 64-column blocks, of the split (fewer blocks than CTAs, slices of unequal length) and of the rows."""
+"""The projection kernel that splits K over a cluster, forced for every shape and split (a shape outside its domain is then an
+error): edges of its tiles (128 rows of W, 64 pairs), of its 64-column blocks, of the split (fewer blocks than CTAs, slices of
+unequal length), of the rows, and more tiles than clusters with 8 and with 16 rows."""
 import numpy as np
 import pytest
 
@@ -18,7 +19,7 @@ def cluster(b200p, request):
 
 
 # the last one has more tiles than clusters and more columns than the two other kernels hold
-@pytest.mark.parametrize("M,N,K", [(1, 128, 512), (2, 130, 528), (3, 65, 1040), (5, 257, 1600), (8, 127, 576), (9, 200, 2048), (16, 96, 544), (13, 2048, 5632), (16, 19400, 8192)])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 512), (4, 70, 16), (12, 140, 144), (2, 130, 528), (3, 65, 1040), (5, 257, 1600), (8, 127, 576), (9, 200, 2048), (16, 96, 544), (13, 2048, 5632), (16, 19400, 8192), (7, 40100, 1024)])
 def test_all_prologues_and_plain_epilogues(b200p, torch_cuda, cluster, M, N, K):
     torch, kind = torch_cuda, "f16" if M == 5 else "bf16"
     rng = np.random.default_rng(M * 1000 + K)
@@ -77,3 +78,12 @@ def test_products_of_one_sign_are_not_truncated_in_long_chains(b200p, torch_cuda
     # two truncated additions lose at most 2^-23 of the sum each; the fp32 sums after them round to nearest, which averages
     # out, below 2^-24.  One accumulator for all of K = 4096: 256 truncations, 5e-6.
     assert ((out.double() - ref).norm() / ref.norm()).item() < 2 * 2.0 ** -23 + 2.0 ** -24
+
+
+def test_a_shape_outside_the_kernel_is_refused_when_it_is_forced(b200p, torch_cuda, cluster):
+    torch = torch_cuda
+    K = 64 * 1100                                            # 8 CTAs: 138 blocks of 8 rows, more than lie beside the ring
+    W, X = torch.zeros((16, K), device="cuda").bfloat16(), torch.zeros((8, K), device="cuda").bfloat16()
+    with pytest.raises(b200p.B200PError) as e:
+        b200p.skinny_gemm(W, torch.zeros((8, 16), device="cuda"), x16=X, epilogue="acc32")
+    assert e.value.status == -10

@@ -395,6 +395,8 @@ def merge_lse_packed(gathered, rows: int, D: int, out):
 
 def workspace_status(workspace) -> int:
     """0, or B200P_E_TIMEOUT if a kernel using this workspace abandoned a bounded wait (synchronises)."""
+    if not workspace.is_cuda:
+        raise ValueError("workspace must be a CUDA tensor: there is no CPU path")
     return int(lib().b200p_attn_workspace_status(workspace.data_ptr(), _stream(workspace)))
 
 

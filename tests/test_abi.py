@@ -65,3 +65,10 @@ def test_cpp_api_header_compiles_and_links(b200p, tmp_path):
                     "-Wl,-rpath," + lib_dir, "-o", str(exe)], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_workspace_status_takes_no_host_memory(b200p):
+    """Like every other call: a CPU tensor is an error before its address reaches the library."""
+    import torch
+    with pytest.raises(ValueError):
+        b200p.workspace_status(torch.zeros(64, dtype=torch.uint8))

@@ -20,7 +20,7 @@
 // instead of the reference's LDS accumulator.
 // These kernels exist for parity with the reference's steps and to exercise the
 // primitives in a simple setting; at the reference's config
-// (0.54 GFLOP, 4 MiB) they are launch-bound on a B200.
+// (0.54 GFLOP, 4 MiB) shared memory bounds them (below).
 // ---------------------------------------------------------------------------
 #include "common.cuh"
 #include "attn_common.cuh"
@@ -408,9 +408,8 @@ extern "C" int b200p_fa_step(int step, int dtype, const void* Q, const void* K, 
         // Lengths off the Br = 16 / Bc = 64 tiling: fp32 I/O takes any seq_len like the reference's fp32 kernels, whose running
         // max starts at the lowest float (kernels/fa_naive.hip:158-169); the 16-bit steps keep the reference's tiling.
         if (dtype != B200P_F32 || seq_q != seq_k) return B200P_E_LENGTH;
-        if ((long long)batch * heads > 65535) return B200P_E_RANGE;
+        if ((long long)batch * heads > 65535) return B200P_E_RANGE;      // as in b200p_fa_rows_f32, the other entry for such lengths
         m_first = -3.402823466e+38f;
-        if (step == 2) step = 1;                           // the reference has no asynchronous form of those
     }
     switch (dtype) {
         case B200P_F16:  return launch_step_d<__half>(step, D, Q, K, V, O, batch, heads, seq_q, seq_k, scale, m_first, st);

@@ -204,3 +204,38 @@ def test_values_behind_a_rows_position_do_not_reach_it(b200p, torch_cuda, batch,
         v2 = v.clone(); v2[:, :, S - 3:] = bad
         first = (S - 3) // 128 * 128                                 # rows that share a tile of keys with the bad ones may see 0 x bad
         assert torch.equal(b200p.prefill(q, k, v2, causal=True)[:, :, :first], clean[:, :, :first])
+
+
+# rows wider than the head, other pitches for O than for Q, other lengths of Q and K: the heads of a group still follow one
+# another, so that they can be one run of rows; and token-major rows, where they cannot
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("D,batch,heads,kv,seqQ,seqK,q_pitch,o_pitch", [
+    (64, 2, 8, 2, 77, 200, 80, 64), (64, 1, 32, 4, 555, 130, 64, 72), (128, 2, 6, 2, 130, 700, 136, 160), (64, 2, 4, 1, 1, 300, 72, 64), (128, 1, 8, 1, 300, 1, 128, 128), (64, 2, 8, 4, 96, 96, 0, 0)])
+def test_packed_rows_of_strided_views(b200p, torch_cuda, causal, D, batch, heads, kv, seqQ, seqK, q_pitch, o_pitch):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(seqQ)
+    if q_pitch:
+        view = lambda t: t[..., :D]
+        qb, shape = torch.randn((batch, heads, seqQ, q_pitch), device="cuda", generator=g).bfloat16(), (batch, heads, seqQ, o_pitch)
+    else:                                                                  # [batch, seq, heads, D]
+        view = lambda t: t.transpose(1, 2)
+        qb, shape = torch.randn((batch, seqQ, heads, D), device="cuda", generator=g).bfloat16(), (batch, seqQ, heads, D)
+    k, v = (torch.randn((batch, kv, seqK, D), device="cuda", generator=g).bfloat16() for _ in range(2))
+    outs = []
+    try:
+        for variant in (16, 20, 24, 28, -1):                     # as in test_work_items_of_every_form_give_the_same_bits
+            b200p.set_tuning("prefill_variant", variant)
+            ob = torch.full(shape, 7.0, device="cuda").bfloat16()
+            b200p.prefill_strided(view(qb), k, v, view(ob), causal=causal)
+            outs.append(ob)
+    finally:
+        b200p.set_tuning("prefill_variant", -1)
+    for o in outs[1:]:
+        assert torch.equal(o, outs[0])
+    if q_pitch:
+        assert (outs[0][..., D:] == 7.0).all()
+    qd, kd, vd = view(qb).double(), k.double().repeat_interleave(heads // kv, 1), v.double().repeat_interleave(heads // kv, 1)
+    s = qd @ kd.transpose(-1, -2) * D ** -0.5
+    if causal:
+        s = s.masked_fill(torch.ones(seqQ, seqK, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    assert (view(outs[0]).double() - s.softmax(-1) @ vd).abs().max() < 2e-2      # 16-bit weights and outputs of size up to 4

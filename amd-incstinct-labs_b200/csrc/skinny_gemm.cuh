@@ -42,7 +42,7 @@
 // the MMA), and skinny_stream_kernel further down, the default, in which a producer
 // thread stages W through a shared-memory ring so that loads run ahead across row
 // groups and the bytes in flight are not bounded by registers.
-// skinny_tc.cuh has a third form, for 9 to 16 rows and for rows too long for one CTA, and the choice between the three.
+// skinny_tc.cuh has a third form, for rows of X that leave these kernels no ring of weights, and the choice between the three.
 // ---------------------------------------------------------------------------
 #pragma once
 #include "common.cuh"

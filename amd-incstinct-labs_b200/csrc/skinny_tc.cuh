@@ -26,13 +26,15 @@
 //    products of the next tile begin under the exchange of this one.
 // What bounds it: the stream of W (HBM), and for one or two tiles per cluster the chain dependency wait -> X -> last
 // stage's products -> exchange -> epilogue.  The shared memory is kept below half an SM's where the ring allows, so that the
-// next kernel's CTAs are resident and fetch their first stages under this one (the decode step: 15.6 -> 14.8 ms).
+// next kernel's CTAs are resident and fetch their first stages under this one (prompt and tokens of 8 layers of width 2048, 16
+// sequences: 15.6 -> 14.8 ms).
 //
 // An inbox buffer is written again only after its owner has read it: a CTA pushes tile i+2 after its own inbox of
 // tile i+1 is complete, which holds parts that the owner pushed after all its warps had read tile i (worker barrier).
 // Waits are bounded.  A wait that gives up raises the abort word, and the thread goes on without waiting, so every
-// thread reaches the worker barriers and the cluster barrier at the end; nobody leaves while a peer may still write
-// to its shared memory.
+// thread reaches the worker barriers and the cluster barrier at the end.  Where every wait succeeded nobody leaves while
+// a peer may still write to its shared memory: each st.async was waited for by its receiver.  After a wait that gave up,
+// one that is still on its way is not waited for; the launch has failed by then and says so in the status word.
 // ---------------------------------------------------------------------------
 #pragma once
 #include "skinny_gemm.cuh"

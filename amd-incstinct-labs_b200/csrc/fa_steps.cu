@@ -55,7 +55,7 @@ template <> __device__ __forceinline__ float exp_for<__nv_bfloat16>(float x) { r
 // the eight lanes of a shared-memory phase hit eight different bank groups.  (Four rows per warp read less but leave too
 // few warps: within 10 % at 8 heads x 512 keys either way.)  Before and after: 8 heads of 64, 512 keys, fp32, step 1
 // 57.7 -> 38.0 us, step 2 54.6 -> 34.6 (its copies were bulk copies behind an mbarrier and an abort word to clear); 12 heads, 333 keys,
-// fp32, which went to the one-row kernels: 110.6 -> 29.2; 24 heads of 128, 1024 keys, fp16: 675 -> 505.
+// fp32, which went to the one-row kernels: step 1 110.6 -> 29.2; 24 heads of 128, 1024 keys, fp16: 675 -> 505.
 // Lengths need not be multiples of the tiles: keys past the end get no weight, rows past the end are not stored.
 constexpr int kRowsPerWarp = 2, kStepThreads = kBr / kRowsPerWarp * 32;
 template <typename T, int D> struct StepTile {
@@ -410,6 +410,9 @@ extern "C" int b200p_fa_step(int step, int dtype, const void* Q, const void* K, 
         if (dtype != B200P_F32 || seq_q != seq_k) return B200P_E_LENGTH;
         if ((long long)batch * heads > 65535) return B200P_E_RANGE;      // as in b200p_fa_rows_f32, the other entry for such lengths
         m_first = -3.402823466e+38f;
+        // Two buffers of 128 fp32 columns leave an SM one CTA: 8 heads, 333 keys, step 1 47.6 us, step 2 52.8; 2 x 12 heads 92.1 and
+        // 104.0.  There step 2 runs step 1 (same bits).  With 64 columns step 2 is the faster one: 28.8 and 26.3 us.
+        if (step == 2 && D == 128) step = 1;
     }
     switch (dtype) {
         case B200P_F16:  return launch_step_d<__half>(step, D, Q, K, V, O, batch, heads, seq_q, seq_k, scale, m_first, st);

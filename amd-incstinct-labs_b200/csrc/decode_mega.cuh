@@ -180,6 +180,7 @@ __device__ __forceinline__ void stream_consume(const SkinnyArgs& a, const Stream
             for (int s = 0; s < 4; ++s) { acc[mh][s][0] = acc[mh][s][1] = acc[mh][s][2] = acc[mh][s][3] = 0.f; }
         EpiAhead<MH> ahead;
         skinny_epilogue_fetch<T, EPI, 2, MH>(a, grp, threadIdx.x, ahead);
+        skinny_epilogue_fetch_constants<T, EPI, MH>(a, grp, threadIdx.x, ahead);
         for (int sl = 0; sl < nslab; ++sl) {
             if (ok && !dme::wait(&r.full_bar[rp.stage], rp.phase, status)) ok = false;
             const int c0 = sl * slab, cols = min(slab, K - c0);

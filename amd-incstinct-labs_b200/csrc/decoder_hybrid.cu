@@ -307,25 +307,34 @@ int layers_step(b200p_session* s, int pos0, cudaStream_t st, const int* pos_dev)
         ++s->gemm_calls;
         return a;
     };
-    // x += X . W^T with rows of X that may be too long for the streaming kernel's shared memory
-    auto add = [&](const void* X, const void* W, int K) -> int {
+    // x += X . W^T with rows of X that may be too long for the streaming kernel's shared memory, and the next norm's input
+    const bool folded = s->fold_parts > 0;
+    auto add = [&](const void* X, const void* W, int K, const void* next_norm) -> int {
         SkinnyArgs a = args(W, s->hidden, H, K, H);
         a.X16 = X; a.ldx = K;
-        const int e = launch_skinny<T, PRO_PLAIN, EPI_ACC32>(a, st);
+        if (folded) write_folded(s, a, next_norm);
+        const int e = folded ? launch_skinny<T, PRO_PLAIN, EPI_ADD_FOLD>(a, st, &s->fold_parts) : launch_skinny<T, PRO_PLAIN, EPI_ACC32>(a, st);
         if (e != B200P_E_RANGE) return e;
         --s->gemm_calls;
-        return session_gemm(s, X, W, s->hidden, M, H, K, K, H, true, true, st);
+        if (int g = session_gemm(s, X, W, s->hidden, M, H, K, K, H, true, true, st)) return g;
+        return folded ? fold_rows(s, next_norm, st) : B200P_OK;
     };
+    // the weights of the norm that reads x after pass p
+    auto norm_after = [&](size_t p) { return p + 1 < L->spec.passes.size() ? L->w[size_t(L->spec.passes[p + 1].layer)].norm1 : s->final_norm; };
     s->final_x = s->hidden;
     for (size_t p = 0; p < L->spec.passes.size(); ++p) {
         const int li = L->spec.passes[p].layer;
         const HybridLayer& ly = L->spec.layers[size_t(li)];
         const HybridWeights& w = L->w[size_t(li)];
-        if (L->spec.passes[p].embed_again) if (int e = embed_again(s, M, st)) return e;
+        if (L->spec.passes[p].embed_again) {
+            if (int e = embed_again(s, M, st)) return e;
+            if (folded) if (int e = fold_rows(s, w.norm1, st)) return e;
+        }
         const int rows = ly.main_row() + ly.ab_row();
         SkinnyArgs a = args(w.proj, L->proj32, rows, H, rows);
         a.X32 = s->hidden; a.norm_w = w.norm1;
-        if (int e = launch_skinny<T, PRO_RMSNORM, EPI_STORE32>(a, st)) return e;
+        if (folded) read_folded(s, a);
+        if (int e = folded ? launch_skinny<T, PRO_SCALED, EPI_STORE32>(a, st) : launch_skinny<T, PRO_RMSNORM, EPI_STORE32>(a, st)) return e;
         if (ly.type->delta) {
             DeltaArgs d = delta_args(s, p, 1, pos0, pos_dev);
             d.proj = L->proj32; d.proj_dtype = B200P_F32; d.ldp = d.ld_ab = rows; d.ab = L->proj32 + ly.main_row();
@@ -335,13 +344,14 @@ int layers_step(b200p_session* s, int pos0, cudaStream_t st, const int* pos_dev)
             g.proj = L->proj32;
             if (int e = grouped_step(g, st)) return e;
         }
-        if (int e = add(L->attn, w.o, ly.v_row())) return e;
+        if (int e = add(L->attn, w.o, ly.v_row(), ly.ff ? w.norm2 : norm_after(p))) return e;
         if (!ly.ff) continue;
         const int F = pad16(ly.ff);
         a = args(w.gu, L->act, F, H, F);
         a.X32 = s->hidden; a.norm_w = w.norm2;
-        if (int e = launch_skinny<T, PRO_RMSNORM, EPI_SILU16>(a, st)) return e;
-        if (int e = add(L->act, w.down, F)) return e;
+        if (folded) read_folded(s, a);
+        if (int e = folded ? launch_skinny<T, PRO_SCALED, EPI_SILU16>(a, st) : launch_skinny<T, PRO_RMSNORM, EPI_SILU16>(a, st)) return e;
+        if (int e = add(L->act, w.down, F, norm_after(p))) return e;
     }
     return B200P_OK;
 }
@@ -350,6 +360,7 @@ template <typename T>
 int hybrid_run_layers(b200p_session* s, int Tn, int pos0, cudaStream_t st, const int* pos_dev) {
     if (!std::is_same_v<T, float> && Tn == 1 && step_ok(s, s->batch)) return layers_step(s, pos0, st, pos_dev);
     if (pos_dev) pos0 = s->kv_len;
+    s->fold_parts = 0;
     return layers_gemm<T>(s, Tn, pos0, st);
 }
 
@@ -484,6 +495,7 @@ int hybrid_build(b200p_session* s, const b200p_model* m) {
     if (int rc = s->dtype == B200P_F32 ? build_weights<float>(s, m) : build_weights<__nv_bfloat16>(s, m)) return rc;
     s->skinny_max_k = L->H;
     s->skinny_usable = s->dtype != B200P_F32;
+    if (s->skinny_usable && s->batch <= kSkinnyMaxM && !L->spec.passes.empty()) s->fold_first = L->w[size_t(L->spec.passes[0].layer)].norm1;
     if (cudaError_t e = s->alloc(&s->d_attn_status, 16)) return int(e);
     return int(cudaMemset(s->d_attn_status, 0, 16));
 }

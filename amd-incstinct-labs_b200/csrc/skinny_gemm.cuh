@@ -57,11 +57,15 @@
 namespace b200p {
 
 enum SkinnyPrologue { PRO_PLAIN = 0, PRO_RMSNORM = 1,
-                      PRO_POSTADD = 2 };         // X = x + RMSNorm(y) * w in fp32, kept for the next reader and rounded to 16 bits (y null: X = x)
+                      PRO_POSTADD = 2,           // X = x + RMSNorm(y) * w in fp32, kept for the next reader and rounded to 16 bits (y null: X = x)
+                      PRO_SCALED = 3 };          // X = x * w rounded to 16 bits by whoever made x; 1 / rms(x) multiplies the products (fp32)
+// X arrives as 16-bit rows that are copied as they are.
+constexpr bool pro_rows16(int pro) { return pro == PRO_PLAIN || pro == PRO_SCALED; }
 enum SkinnyEpilogue { EPI_STORE16 = 0, EPI_ACC32 = 1, EPI_STORE32 = 2, EPI_SILU16 = 3, EPI_ROPE = 4,
                       EPI_STORE32_BEST = 5,      // fp32 store + running argmax key per row (decode_mega.cuh only)
                       EPI_GELU16 = 6,            // like EPI_SILU16 with the tanh form of GELU
-                      EPI_PAIRROT = 7 };         // queries whose heads are [plain | rotated] parts (SkinnyPairRot)
+                      EPI_PAIRROT = 7,           // queries whose heads are [plain | rotated] parts (SkinnyPairRot)
+                      EPI_ADD_FOLD = 8 };        // EPI_ACC32, and what a PRO_SCALED reader of the sum needs (SkinnyFold)
 // Gated epilogues: W is [2N][K], gate rows then up rows; out = act(gate) * up.
 constexpr bool epi_gated(int epi) { return epi == EPI_SILU16 || epi == EPI_GELU16; }
 // A group's rows g and g + 8 meet in one thread.
@@ -101,6 +105,20 @@ struct SkinnyPairRot {
     int pos0, Tn, plain, rotated, heads, rot_ld, rot_col, max_seq;
 };
 
+// The residual stream x as the next norm's reader takes it: x * w in 16 bits, and sums of squares of x.  A norm ahead of a
+// projection is W . (x * inv * w) = inv * (W . (x * w)) with one inv per row, so whoever adds to x (EPI_ADD_FOLD: each CTA
+// its columns) rounds x * w once for all readers, and a reader copies 16-bit rows and scales its sums.  As a prologue
+// (PRO_RMSNORM) every CTA reads all of x in fp32 and, from eight rows on, goes through it twice.  Decode step of 22 layers of width
+// 2048, 2 / 8 / 16 sequences: 0.576 / 0.737 / 0.998 ms with the prologues, 0.560 / 0.597 / 0.803 folded; 8 layers of width 4096, 2 sequences: 0.685, 0.644.  The rounding is the same size: one 16-bit rounding per operand, whose exponent does not matter to
+// bf16; fp16 could overflow ahead of the scale, so fp16 sessions keep the prologue.
+struct SkinnyFold {
+    const float* ss;       // PRO_SCALED: [M][ss_ld] sums of squares of a row over disjoint columns, `parts` of them
+    int parts, ss_ld;
+    const void* w;         // EPI_ADD_FOLD: weights [N] of the norm that reads next
+    void* x16;             //               [M][N] 16-bit
+    float* ss_out;         //               [M][ss_ld]: as many parts as the launcher says
+};
+
 struct SkinnyArgs {
     const void*  W;        // [N][K] 16-bit (EPI_SILU16: [2N][K], gate rows then up rows)
     const void*  X16;      // PRO_PLAIN:   [M][ldx] 16-bit activations
@@ -117,6 +135,7 @@ struct SkinnyArgs {
     float* x_out;          // PRO_POSTADD with Y32: [M][K] fp32, the sum (another buffer than X32)
     SkinnyRope rope;       // EPI_ROPE only
     SkinnyPairRot pair;    // EPI_PAIRROT only
+    SkinnyFold fold;       // PRO_SCALED, EPI_ADD_FOLD
     int* abort_word;       // streaming kernel: the abort word its bounded waits poll and raise.  A caller that
                            // launches many of these on one stream (the runtime's decode step) owns one word,
                            // clears it before the step and reads it after; null: a per-launch slot is taken.
@@ -345,7 +364,49 @@ template <int MH>
 struct EpiAhead {
     float prev[MH];
     float c, sn, b0, b1;
+    float add;                 // EPI_ADD_FOLD: residual value ...
+    unsigned short fw;         // ... and the next norm's weight, 16 bits as loaded: a conversion here would wait for the load
 };
+// Row and column of X of a thread in EPI_ADD_FOLD (128 threads per eight rows): lanes l, l ^ 4, l ^ 8, l ^ 16 share the row, and a
+// warp's eight columns are one partial sum.
+__device__ __forceinline__ int fold_row(int tid) { return 8 * (tid / 128) + 2 * (tid % 4) + (tid / 32) % 2; }
+__device__ __forceinline__ int fold_part(int grp, int tid) { return grp * 2 + (tid / 64) % 2; }
+__device__ __forceinline__ int fold_col(int grp, int tid) { return fold_part(grp, tid) * 8 + (tid % 32) / 4; }
+
+// 1 / rms of the rows of X from the partial sums, in the same order in every CTA and call, a warp for rows warp and warp + 8:
+// fold_load asks for a row's first 128 * VECS sums, fold_inverse adds up, after the products; inv [M] is there after the next
+// barrier of the computing threads.
+template <int MH, int VECS>
+__device__ __forceinline__ void fold_load(const SkinnyArgs& a, int warp, int lane, float4 (&v)[MH][VECS]) {
+    #pragma unroll
+    for (int r = 0; r < MH; ++r) {
+        const int m = warp + kSkinnyWarps * r, parts = m < a.M ? a.fold.parts : 0;
+        const float* src = a.fold.ss + size_t(m) * a.fold.ss_ld + 4 * lane;      // (ss_ld is a multiple of 16: a vector ends inside the row)
+        #pragma unroll
+        for (int u = 0; u < VECS; ++u) {
+            v[r][u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (4 * lane + 128 * u < parts) v[r][u] = *reinterpret_cast<const float4*>(src + 128 * u);
+        }
+    }
+}
+template <int MH, int VECS>
+__device__ __forceinline__ void fold_inverse(const SkinnyArgs& a, int warp, int lane, const float4 (&v)[MH][VECS], float* inv) {
+    #pragma unroll
+    for (int r = 0; r < MH; ++r) {
+        const int m = warp + kSkinnyWarps * r, parts = a.fold.parts;
+        if (m >= a.M) break;
+        float s = 0.f;
+        #pragma unroll
+        for (int u = 0; u < VECS; ++u) {
+            const int p = 4 * lane + 128 * u;                     // what lies past `parts` is another kernel's
+            s += ((p < parts ? v[r][u].x : 0.f) + (p + 1 < parts ? v[r][u].y : 0.f)) + ((p + 2 < parts ? v[r][u].z : 0.f) + (p + 3 < parts ? v[r][u].w : 0.f));
+        }
+        for (int p = lane + 128 * VECS; p < parts; p += 32) s += a.fold.ss[size_t(m) * a.fold.ss_ld + p];
+        s = wave::dpp::reduce_sum(s);
+        if (lane == 0) inv[m] = rsqrtf(s / float(a.norm_n ? a.norm_n : a.K) + a.eps);
+    }
+}
+
 template <typename T, int EPI, int R, int MH>
 __device__ __forceinline__ void skinny_epilogue_fetch(const SkinnyArgs& a, int grp, int tid, EpiAhead<MH>& e) {
     if (EPI == EPI_ACC32) {
@@ -357,6 +418,22 @@ __device__ __forceinline__ void skinny_epilogue_fetch(const SkinnyArgs& a, int g
                 const int m = 8 * mh + 2 * (l % 4) + (c & 1);
                 e.prev[mh] = (m < a.M && n < a.N) ? static_cast<const float*>(a.out)[size_t(m) * a.ldo + n] : 0.f;
             }
+        }
+    } else if (EPI == EPI_ADD_FOLD) {
+        if (tid < 128 * MH) {
+            const int m = fold_row(tid), n = fold_col(grp, tid);
+            e.add = m < a.M && n < a.N ? static_cast<const float*>(a.out)[size_t(m) * a.ldo + n] : 0.f;
+        }
+    }
+}
+// The part that no earlier kernel of the step writes: weights, tables, and the position, which is set by launches that have completed
+// before a step's first kernel, an ordinary launch, starts.  May run ahead of the dependency wait.
+template <typename T, int EPI, int MH>
+__device__ __forceinline__ void skinny_epilogue_fetch_constants(const SkinnyArgs& a, int grp, int tid, EpiAhead<MH>& e) {
+    if (EPI == EPI_ADD_FOLD) {
+        if (tid < 128 * MH) {
+            const int n = fold_col(grp, tid);
+            e.fw = n < a.N ? static_cast<const unsigned short*>(a.fold.w)[n] : 0;
         }
     } else if (EPI == EPI_ROPE) {
         if (tid < 64) {
@@ -374,6 +451,7 @@ __device__ __forceinline__ void skinny_epilogue_fetch(const SkinnyArgs& a, int g
         }
     }
 }
+template <typename T> __device__ __forceinline__ float raw_float(unsigned short v) { return to_float(*reinterpret_cast<const T*>(&v)); }
 
 // Position and table offset of pair j of row m (EPI_PAIRROT).
 __device__ __forceinline__ size_t pair_angle(const SkinnyPairRot& r, int m, int j) {
@@ -382,9 +460,26 @@ __device__ __forceinline__ size_t pair_angle(const SkinnyPairRot& r, int m, int 
 }
 
 // red[warp][lane][4 * mh + c]: the m16n8 C fragment of the MMA over rows 8 mh .. 8 mh + 7 of X.
-template <typename T, int EPI, int R, int MH>
+template <typename T, int EPI, int R, int MH, bool SCALED = false>
 __device__ __forceinline__ void skinny_epilogue(const SkinnyArgs& a, const float (*red)[32][4 * MH], int grp, int tid, bool use_prev, float prev,
-                                                unsigned long long* best = nullptr, const EpiAhead<MH>* ahead = nullptr) {
+                                                unsigned long long* best = nullptr, const EpiAhead<MH>* ahead = nullptr, const float* inv = nullptr) {
+    if constexpr (EPI == EPI_ADD_FOLD) {
+        if (tid < 128 * MH) {                                    // whole warps
+            const int l = tid % 32, c = tid / 32 % 4, m = fold_row(tid), n = fold_col(grp, tid);
+            float v = 0.f, ss = 0.f;
+            #pragma unroll
+            for (int w = 0; w < kSkinnyWarps; ++w) v += red[w][l][4 * (tid / 128) + c];
+            if (m < a.M && n < a.N) {
+                const float x = ahead->add + v;
+                static_cast<float*>(a.out)[size_t(m) * a.ldo + n] = x;
+                static_cast<T*>(a.fold.x16)[size_t(m) * a.N + n] = from_float<T>(x * raw_float<T>(ahead->fw));
+                ss = x * x;
+            }
+            #pragma unroll
+            for (int off = 4; off < 32; off *= 2) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+            if (l < 4 && m < a.M) a.fold.ss_out[size_t(m) * a.fold.ss_ld + fold_part(grp, tid)] = ss;
+        }
+    } else {
     #pragma unroll
     for (int mh = 0; mh < MH; ++mh) {
         if (epi_gated(EPI)) {
@@ -393,6 +488,7 @@ __device__ __forceinline__ void skinny_epilogue(const SkinnyArgs& a, const float
                 float gate = 0.f, up = 0.f;
                 #pragma unroll
                 for (int w = 0; w < kSkinnyWarps; ++w) { gate += red[w][l][4 * mh + sel]; up += red[w][l][4 * mh + 2 + sel]; }
+                if (SCALED) { const float c = inv[8 * mh + 2 * (l % 4) + sel]; gate *= c; up *= c; }
                 const int m = 8 * mh + 2 * (l % 4) + sel, p = grp * 8 + l / 4;
                 if (m < a.M && p < a.N)
                     static_cast<T*>(a.out)[size_t(m) * a.ldo + p] = from_float<T>(gate_act<EPI>(gate) * up);
@@ -404,6 +500,7 @@ __device__ __forceinline__ void skinny_epilogue(const SkinnyArgs& a, const float
                 float x0 = 0.f, x1 = 0.f;
                 #pragma unroll
                 for (int w = 0; w < kSkinnyWarps; ++w) { x0 += red[w][l][4 * mh + sel]; x1 += red[w][l][4 * mh + 2 + sel]; }
+                if (SCALED) { const float c = inv[8 * mh + 2 * (l % 4) + sel]; x0 *= c; x1 *= c; }
                 const int m = 8 * mh + 2 * (l % 4) + sel;
                 if (m < a.M) {
                     const int cph = r.D / 16, half = r.D / 2;
@@ -439,6 +536,7 @@ __device__ __forceinline__ void skinny_epilogue(const SkinnyArgs& a, const float
                 float x0 = 0.f, x1 = 0.f;
                 #pragma unroll
                 for (int w = 0; w < kSkinnyWarps; ++w) { x0 += red[w][l][4 * mh + sel]; x1 += red[w][l][4 * mh + 2 + sel]; }
+                if (SCALED) { const float c = inv[8 * mh + 2 * (l % 4) + sel]; x0 *= c; x1 *= c; }
                 const int m = 8 * mh + 2 * (l % 4) + sel;
                 const int per_head = r.plain + r.rotated, head = grp * 16 / per_head, j = grp * 16 % per_head;
                 if (m < a.M && head < r.heads) {
@@ -458,6 +556,7 @@ __device__ __forceinline__ void skinny_epilogue(const SkinnyArgs& a, const float
             float v = 0.f;
             #pragma unroll
             for (int w = 0; w < kSkinnyWarps; ++w) v += red[w][l][4 * mh + c];
+            if (SCALED) v *= inv[8 * mh + 2 * (l % 4) + (c & 1)];
             const int m = 8 * mh + 2 * (l % 4) + (c & 1), n = grp * 8 * R + l / 4 + 8 * (c >> 1);
             if (m < a.M && n < a.N) {
                 const size_t idx = size_t(m) * a.ldo + n;
@@ -477,6 +576,7 @@ __device__ __forceinline__ void skinny_epilogue(const SkinnyArgs& a, const float
                 else                         static_cast<float*>(a.out)[idx] += v;
             }
         }
+    }
     }
 }
 
@@ -622,15 +722,17 @@ skinny_gemm_kernel(const SkinnyArgs a) {
 // ---------------------------------------------------------------------------
 constexpr int kSkinnySlab = 2048;                  // columns of W per stage
 constexpr int kSkinnyStreamThreads = kSkinnyThreads + 32;
+constexpr int kSkinnyXBars = 4;                    // barriers of the copies of X
 
 template <typename T, int PRO, int EPI, int MH>
-__global__ void __launch_bounds__(kSkinnyStreamThreads, 1)
+__global__ void __launch_bounds__(kSkinnyStreamThreads, EPI == EPI_ROPE && MH == 1 ? 2 : 1)
 skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status, int* sticky) {
     griddep_launch_dependents();
     extern __shared__ __align__(128) unsigned char skinny_smem[];
     __shared__ float red[2][kSkinnyWarps][32][4 * MH];
     __shared__ __align__(16) float part_ss[kSkinnyWarps];
-    __shared__ uint64_t bars[16];
+    __shared__ float inv_rms[PRO == PRO_SCALED ? 8 * MH : 1];
+    __shared__ uint64_t bars[16], x_bar[kSkinnyXBars];
     constexpr int kMaxStages = 8;
     uint64_t* full_bar = bars;
     uint64_t* empty_bar = bars + kMaxStages;
@@ -646,13 +748,16 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
     unsigned char* stages = skinny_smem + x_bytes;
     const int ngroups = (epi_gated(EPI)) ? (a.N + 7) / 8 : (a.N + 15) / 16;
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < nstages; ++s) { dme::mbar_init(&full_bar[s], 1); dme::mbar_init(&empty_bar[s], kSkinnyWarps); }
-        dme::mbar_init_fence();
-    }
-    __syncthreads();
-
+    // A CTA often starts when the last CTA of the kernel before leaves its SM, and what precedes the dependency wait is then part of
+    // the chain: the producer sets up the barriers and streams, the others go to the wait at once and meet it (barrier 2) afterwards.
     if (warp == kSkinnyWarps) {
+        if (lane == 0) {
+            for (int s = 0; s < nstages; ++s) { dme::mbar_init(&full_bar[s], 1); dme::mbar_init(&empty_bar[s], kSkinnyWarps); }
+            for (int s = 0; s < kSkinnyXBars; ++s) dme::mbar_init(&x_bar[s], 1);
+            dme::mbar_init_fence();
+        }
+        __syncwarp();
+        asm volatile("bar.arrive 2, %0;" :: "n"(kSkinnyStreamThreads) : "memory");
         // ---- producer: W is constant, so it streams before and through the dependency wait of the consumers ----
         if (lane == 0) {
             const uint64_t pol = dme::policy_evict_first();
@@ -664,6 +769,7 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
                     const int c0 = sl * slab, cols = min(slab, K - c0);
                     unsigned char* dst = stages + size_t(stage) * stage_bytes;
                     dme::mbar_arrive_expect_tx(&full_bar[stage], uint32_t(16 * cols * 2));
+                    #pragma unroll 2
                     for (int r = 0; r < 16; ++r) {
                         size_t row;
                         if (epi_gated(EPI))    row = r < 8 ? size_t(min(grp * 8 + r, a.N - 1)) : size_t(a.N) + size_t(min(grp * 8 + r - 8, a.N - 1));
@@ -681,8 +787,29 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
     } else {
         // ---- consumers ------------------------------------------------------------------------------------------
         const int g = lane / 4, t4 = lane % 4;
+        EpiAhead<MH> ahead;
+        float4 sums[PRO == PRO_SCALED ? MH : 1][EPI == EPI_ROPE ? 2 : 4];
+        if (EPI != EPI_ROPE) skinny_epilogue_fetch_constants<T, EPI, MH>(a, blockIdx.x, threadIdx.x, ahead);
+        asm volatile("bar.sync 2, %0;" :: "n"(kSkinnyStreamThreads) : "memory");       // the mbarriers are there
+        // 16-bit rows of X: one bulk copy per row and slab (a barrier each for the first slabs, the last for the rest).  Through
+        // registers they came in batches, one trip to L2 after the other (16 rows of 2048: eight, 3.4 us; 1.3 by copies)
+        if (pro_rows16(PRO) && threadIdx.x == 0)
+            for (int b = 0; b < min(nslab, kSkinnyXBars); ++b)
+                dme::mbar_arrive_expect_tx(&x_bar[b], uint32_t(a.M) * uint32_t((b < kSkinnyXBars - 1 ? min(slab, K - b * slab) : K - b * slab) * 2));
         griddep_wait();                                           // activations come from earlier kernels of the stream
-        skinny_prologue<T, PRO>(a, xs, part_ss, Mp, warp, lane);
+        if constexpr (pro_rows16(PRO)) {
+            // (what the kernels before wrote is visible to the copies too once the wait has returned; a fence here took 500 ns)
+            if (warp == 0 && lane < a.M) {
+                const T* src = static_cast<const T*>(a.X16) + size_t(lane) * a.ldx;
+                for (int c0 = 0, b = 0; c0 < K; c0 += slab, b = min(b + 1, kSkinnyXBars - 1))
+                    dme::copy_tile_1d(xs + size_t(lane) * xstride + c0, src + c0, uint32_t(min(slab, K - c0) * 2), &x_bar[b]);
+            }
+            __syncwarp();
+            if constexpr (PRO == PRO_SCALED) fold_load(a, warp, lane, sums);
+        } else {
+            skinny_prologue<T, PRO>(a, xs, part_ss, Mp, warp, lane);
+        }
+        const int rows = pro_rows16(PRO) ? a.M : Mp;              // rows of X in shared memory
         const T* xrow = xs + size_t(g) * xstride + t4 * 16;
         int stage = 0; uint32_t phase = 0;
         int parity = 0;
@@ -696,9 +823,10 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
                 #pragma unroll
                 for (int s = 0; s < 4; ++s) { acc[mh][s][0] = acc[mh][s][1] = acc[mh][s][2] = acc[mh][s][3] = 0.f; }
             }
-            EpiAhead<MH> ahead;
             skinny_epilogue_fetch<T, EPI, 2, MH>(a, grp, threadIdx.x, ahead);
+            if (EPI == EPI_ROPE || grp != int(blockIdx.x)) skinny_epilogue_fetch_constants<T, EPI, MH>(a, grp, threadIdx.x, ahead);
             for (int sl = 0; sl < nslab; ++sl) {
+                if (pro_rows16(PRO) && grp == int(blockIdx.x) && ok && !dme::wait(&x_bar[min(sl, kSkinnyXBars - 1)], 0, status)) ok = false;
                 if (ok && !dme::wait(&full_bar[stage], phase, status)) ok = false;
                 const int c0 = sl * slab, cols = min(slab, K - c0);
                 const int nblk = (cols + 63) / 64;
@@ -706,7 +834,7 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
                 if (ok && cols % (64 * kSkinnyWarps) == 0) {
                     // whole blocks for every warp (the usual stage): nb blocks each, taken BB at a time with every
                     // shared-memory load of the batch issued before its first MMA
-                    constexpr int BB = 4 / MH;
+                    constexpr int BB = EPI == EPI_ROPE ? 2 : 4 / MH;         // Q/K/V: two CTAs share an SM, at most 96 registers
                     const int nb = cols / (64 * kSkinnyWarps);
                     const unsigned char* wrow_a = st + size_t(g) * rowb + t4 * 32;
                     const unsigned char* wrow_b = st + size_t(g + 8) * rowb + t4 * 32;
@@ -721,7 +849,7 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
                             #pragma unroll
                             for (int mh = 0; mh < MH; ++mh) {
                                 xv[b][mh][0] = xv[b][mh][1] = make_uint4(0u, 0u, 0u, 0u);
-                                if (g + 8 * mh < Mp) {
+                                if (g + 8 * mh < rows) {
                                     const uint4* xp = reinterpret_cast<const uint4*>(xrow + size_t(8 * mh) * xstride + c0 + blk * 64);
                                     xv[b][mh][0] = xp[0]; xv[b][mh][1] = xp[1];
                                 }
@@ -759,7 +887,7 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
                         #pragma unroll
                         for (int mh = 0; mh < MH; ++mh) {
                             uint4 xa = make_uint4(0u, 0u, 0u, 0u), xb = xa;
-                            if (live && g + 8 * mh < Mp) {
+                            if (live && g + 8 * mh < rows) {
                                 const uint4* xp = reinterpret_cast<const uint4*>(xrow + size_t(8 * mh) * xstride + c0 + blk * 64);
                                 xa = xp[0]; xb = xp[1];
                             }
@@ -776,14 +904,17 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
                 if (lane == 0) dme::mbar_arrive(&empty_bar[stage]);
                 if (++stage == nstages) { stage = 0; phase ^= 1u; }
             }
+            if constexpr (PRO == PRO_SCALED) if (grp == int(blockIdx.x)) fold_inverse(a, warp, lane, sums, inv_rms);
             #pragma unroll
             for (int mh = 0; mh < MH; ++mh)
                 *reinterpret_cast<float4*>(&red[parity][warp][lane][4 * mh]) =
                     make_float4((acc[mh][0][0] + acc[mh][1][0]) + (acc[mh][2][0] + acc[mh][3][0]), (acc[mh][0][1] + acc[mh][1][1]) + (acc[mh][2][1] + acc[mh][3][1]),
                                 (acc[mh][0][2] + acc[mh][1][2]) + (acc[mh][2][2] + acc[mh][3][2]), (acc[mh][0][3] + acc[mh][1][3]) + (acc[mh][2][3] + acc[mh][3][3]));
             skinny_barrier();
-            skinny_epilogue<T, EPI, 2, MH>(a, red[parity], grp, threadIdx.x, false, 0.f, nullptr, &ahead);
+            skinny_epilogue<T, EPI, 2, MH, PRO == PRO_SCALED>(a, red[parity], grp, threadIdx.x, false, 0.f, nullptr, &ahead, inv_rms);
         }
+        if (!ok && pro_rows16(PRO) && warp == 0)                  // the copies of X land before this CTA's shared memory is given up
+            for (int b = 0; b < min(nslab, kSkinnyXBars); ++b) dme::wait(&x_bar[b], 0);
         if (!ok && lane == 0) atomicExch(sticky, 1);
     }
 }
@@ -794,9 +925,9 @@ inline bool skinny_rows_fit(int M, int K) {
 }
 
 // Launch of shapes in skinny_domain (skinny_tc.cuh, which chooses between these kernels and its own); B200P_E_RANGE: they
-// do not fit these kernels either.
+// do not fit these kernels either.  *parts: EPI_ADD_FOLD's number of partial sums.  The folded forms have no register kernel.
 template <typename T, int PRO, int EPI, int MH>
-int launch_skinny_mh(const SkinnyArgs& a, cudaStream_t st) {
+int launch_skinny_mh(const SkinnyArgs& a, cudaStream_t st, int* parts = nullptr) {
     if (!skinny_rows_fit(a.M, a.K)) return B200P_E_RANGE;
     const int Mp = a.M <= 1 ? 1 : a.M <= 2 ? 2 : a.M <= 4 ? 4 : a.M <= 8 ? 8 : 16;
     const size_t smem = size_t(Mp) * (a.K + kSkinnyXPad) * 2;
@@ -805,11 +936,13 @@ int launch_skinny_mh(const SkinnyArgs& a, cudaStream_t st) {
     const bool pdl = tuning(KNOB_RUNTIME_PDL, 1) != 0;
     if (tuning(KNOB_RUNTIME_SKINNY, 2) == 2 && aligned(a.W, 16)) {
         // W staged through shared memory by a producer thread (skinny_stream_kernel), one CTA per SM
-        const int slab_cols = kSkinnySlab;                               // measured: 0.67 ms per token at 2048, 0.72 at 1024, 0.73 at 4096
+        int slab_cols = kSkinnySlab;                                     // measured: 0.67 ms per token at 2048, 0.72 at 1024, 0.73 at 4096
+        const int x_bytes = int((smem + 127) / 128 * 128);
+        // half a stage where X leaves room for one whole stage only (16 rows of 3072)
+        if (a.K > slab_cols && (223488 - 8192 * (MH - 1) - x_bytes) / (16 * (slab_cols * 2 + 16)) == 1) slab_cols /= 2;
         const int slab = a.K < slab_cols ? a.K : slab_cols;
         const int stage_bytes = 16 * (slab * 2 + 16);
-        const int x_bytes = int((smem + 127) / 128 * 128);
-        int nstages = (224000 - 8192 * (MH - 1) - x_bytes) / stage_bytes;
+        int nstages = (223488 - 8192 * (MH - 1) - x_bytes) / stage_bytes;
         if (nstages > 8) nstages = 8;
         // A few more row groups than SMs (the decode step's Q/K/V: 160 on 148), each one stage long: with one CTA per
         // SM a dozen CTAs would take two groups one after the other and the whole grid would wait for them.  One CTA
@@ -839,9 +972,12 @@ int launch_skinny_mh(const SkinnyArgs& a, cudaStream_t st) {
             cfg.attrs = attr; cfg.numAttrs = pdl ? 1 : 0;
             const cudaError_t le = cudaLaunchKernelEx(&cfg, sk, a, nstages, slab_cols, status, sticky);
             g_launches.fetch_add(1, std::memory_order_relaxed);
+            if (parts) *parts = 2 * groups;
             return le == cudaSuccess ? B200P_OK : int(le);
         }
     }
+    if constexpr (PRO == PRO_SCALED || EPI == EPI_ADD_FOLD) return B200P_E_RANGE;
+    else {
     if (!aligned(a.W, 32)) return B200P_E_RANGE;               // the register kernel loads 32-byte vectors of W
     // 8-row groups when 16-row groups would leave a third of the CTA slots (2 per SM) empty
     const bool half_rows = !paired && (a.N + 15) / 16 < (4 * sms) / 3;
@@ -863,6 +999,7 @@ int launch_skinny_mh(const SkinnyArgs& a, cudaStream_t st) {
     const cudaError_t le = cudaLaunchKernelEx(&cfg, kern, a);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return le == cudaSuccess ? B200P_OK : int(le);
+    }
 }
 
 } // namespace b200p

@@ -154,12 +154,23 @@ LatentState* latent(const b200p_session* s) { return static_cast<LatentState*>(s
 // WPR warps of a CTA share a row: one where there are many rows, all eight in the decode step.
 template <typename T, int WPR>
 __global__ void __launch_bounds__(256)
-postnorm_add_kernel(float* __restrict__ X, const float* __restrict__ Y, const T* __restrict__ W, T* __restrict__ X16, int rows, int H, int n, float eps) {
+postnorm_add_kernel(float* __restrict__ X, const float* __restrict__ Y, const T* __restrict__ W, T* __restrict__ X16, int rows, int H, int n, float eps,
+                    const T* __restrict__ fold_w, float* __restrict__ ss_out, int ss_ld) {
     griddep_launch_dependents();
-    griddep_wait();
-    __shared__ float part[8];
+    __shared__ float part[8], part_x[8];
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32 + 32 * (warp % WPR);
     const int r = blockIdx.x * (8 / WPR) + warp / WPR;
+    // the weights are no kernel's output: the decode step asks for them ahead of the dependency wait
+    constexpr int WCACHE = WPR == 8 && !std::is_same_v<T, float> ? 4 : 0;
+    uint2 cw[WCACHE ? WCACHE : 1], cf[WCACHE ? WCACHE : 1];
+    #pragma unroll
+    for (int i = 0; i < WCACHE; ++i) {
+        const int q = lane + 32 * WPR * i;
+        cw[i] = cf[i] = make_uint2(0u, 0u);
+        if (q < H / 4 && Y) cw[i] = *reinterpret_cast<const uint2*>(W + 4 * q);
+        if (q < H / 4 && fold_w) cf[i] = *reinterpret_cast<const uint2*>(fold_w + 4 * q);
+    }
+    griddep_wait();
     if (r >= rows) return;                                    // (WPR = 8: the whole CTA or nothing)
     float* x = X + size_t(r) * H;
     const float* y = Y ? Y + size_t(r) * H : nullptr;
@@ -185,26 +196,50 @@ postnorm_add_kernel(float* __restrict__ X, const float* __restrict__ Y, const T*
         for (int k = 0; k < WPR; ++k) ss += part[k];
     }
     const float inv = rsqrtf(ss / n + eps);
-    auto put = [&](int q, float4 o, const float4& v) {
+    float xx = 0.f;
+    auto put = [&](int q, float4 o, const float4& v, const T* wp, const T* fp) {
         if (y) {
-            const float4 w = load4<T>(W + 4 * q);
+            const float4 w = load4<T>(wp);
             o.x += v.x * inv * w.x; o.y += v.y * inv * w.y; o.z += v.z * inv * w.z; o.w += v.w * inv * w.w;
             store4<float>(x + 4 * q, o);
         }
-        if (!std::is_same_v<T, float>) store4<T>(X16 + size_t(r) * H + 4 * q, o);
+        if (std::is_same_v<T, float>) return;
+        if (fold_w) {                                         // the last sum: the final norm's folded form (SkinnyFold) instead of x
+            const float4 f = load4<T>(fp);
+            xx += o.x * o.x + o.y * o.y + o.z * o.z + o.w * o.w;
+            o.x *= f.x; o.y *= f.y; o.z *= f.z; o.w *= f.w;
+        }
+        store4<T>(X16 + size_t(r) * H + 4 * q, o);
     };
     #pragma unroll
-    for (int i = 0; i < CACHE; ++i) { const int q = lane + STEP * i; if (q < quads) put(q, WPR > 1 ? xv[WPR == 1 ? 0 : i] : load4<float>(x + 4 * q), c[i]); }
-    for (int q = lane + STEP * CACHE; q < quads; q += STEP) put(q, load4<float>(x + 4 * q), y ? load4<float>(y + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f));
+    for (int i = 0; i < CACHE; ++i) {
+        const int q = lane + STEP * i;
+        const T *wp = WCACHE ? reinterpret_cast<const T*>(&cw[WCACHE ? i : 0]) : W + 4 * q, *fp = WCACHE ? reinterpret_cast<const T*>(&cf[WCACHE ? i : 0]) : fold_w + 4 * q;
+        if (q < quads) put(q, WPR > 1 ? xv[WPR == 1 ? 0 : i] : load4<float>(x + 4 * q), c[i], wp, fp);
+    }
+    for (int q = lane + STEP * CACHE; q < quads; q += STEP) put(q, load4<float>(x + 4 * q), y ? load4<float>(y + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f), W + 4 * q, fold_w + 4 * q);
+    if (WPR > 1 && fold_w) {
+        xx = wave::dpp::reduce_sum(xx);
+        if (threadIdx.x % 32 == 0) part_x[warp] = xx;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            xx = 0.f;
+            #pragma unroll
+            for (int k = 0; k < WPR; ++k) xx += part_x[k];
+            ss_out[size_t(r) * ss_ld] = xx;
+        }
+    }
 }
 
 template <typename T>
-int postnorm_add(float* x, const float* y, const void* w, void* x16, int rows, int H, int n, float eps, cudaStream_t st) {
+int postnorm_add(float* x, const float* y, const void* w, void* x16, int rows, int H, int n, float eps, cudaStream_t st,
+                 const void* fold_w = nullptr, float* ss_out = nullptr, int ss_ld = 0) {
+    const T* none = nullptr;
     if (rows > 64) {
-        postnorm_add_kernel<T, 1><<<blocks(size_t(rows) * 32), 256, 0, st>>>(x, y, static_cast<const T*>(w), static_cast<T*>(x16), rows, H, n, eps);
+        postnorm_add_kernel<T, 1><<<blocks(size_t(rows) * 32), 256, 0, st>>>(x, y, static_cast<const T*>(w), static_cast<T*>(x16), rows, H, n, eps, none, static_cast<float*>(nullptr), 0);
         return launched();
     }
-    return launch_dependent(postnorm_add_kernel<T, 8>, dim3(unsigned(rows)), 256, 0, st, x, y, static_cast<const T*>(w), static_cast<T*>(x16), rows, H, n, eps);
+    return launch_dependent(postnorm_add_kernel<T, 8>, dim3(unsigned(rows)), 256, 0, st, x, y, static_cast<const T*>(w), static_cast<T*>(x16), rows, H, n, eps, static_cast<const T*>(fold_w), ss_out, ss_ld);
 }
 
 struct LatentNormArgs {
@@ -433,6 +468,11 @@ int layers_few(b200p_session* s, int Tn, int pos0, cudaStream_t st, const int* p
         pending = L->y; pending_w = w.norm2;
     }
     s->final_x = x;
+    s->fold_parts = 0;
+    if (Tn == 1 && fold_ok(s)) {                        // one token per sequence: the head reads the final norm's folded form
+        s->fold_parts = 1;
+        return postnorm_add<T>(x, pending, pending_w, s->fold_x16, M, H, n, s->eps, st, s->final_norm, s->fold_ss, fold_parts_most(H));
+    }
     return postnorm_add<T>(x, pending, pending_w, L->x16, M, H, n, s->eps, st);
 }
 
@@ -440,6 +480,7 @@ template <typename T>
 int latent_run_layers(b200p_session* s, int Tn, int pos0, cudaStream_t st, const int* pos_dev) {
     if (!std::is_same_v<T, float> && few_tokens(s, s->batch * Tn)) return layers_few(s, Tn, pos0, st, pos_dev);
     if (pos_dev) pos0 = s->kv_len;
+    s->fold_parts = 0;
     return layers_gemm<T>(s, Tn, pos0, st);
 }
 
@@ -581,6 +622,7 @@ int latent_build(b200p_session* s, const b200p_model* m) {
     }
     s->skinny_max_k = max_k;
     s->skinny_usable = s->dtype != B200P_F32;
+    if (s->skinny_usable && s->batch <= kSkinnyMaxM) s->fold_first = s->final_norm;      // only the head's norm is folded
     if (cudaError_t e = s->alloc(&L->kv, size_t(s->batch) * s->max_seq * L->max_kv * esz)) return int(e);
     if (s->dtype == B200P_BF16) {                         // the absorbed attention's queries and partial results
         size_t parts = 0, part_floats = 0, abs = 0;

@@ -152,7 +152,8 @@ constexpr int kSkinnyXPad = 8;        // elements: X rows are 16 bytes longer th
 __device__ __forceinline__ void skinny_barrier() { asm volatile("bar.sync 1, %0;" :: "r"(kSkinnyThreads) : "memory"); }
 
 // X into shared memory as 16-bit rows of K + kSkinnyXPad elements, rows in [M, Mp) zero; ends with a barrier.
-template <typename T, int PRO, bool EMB = false>
+// HELD: quads of a row that a lane holds between the sum of squares and the scaling (PRO_RMSNORM).
+template <typename T, int PRO, bool EMB = false, int HELD = 4>
 __device__ __forceinline__ void skinny_prologue(const SkinnyArgs& a, T* xs, float* part_ss, int Mp, int warp, int lane) {
     const int K = a.K, xstride = K + kSkinnyXPad;
     // ---- prologue: X into shared memory as 16-bit, rows in [M, Mp) zero --------------------------------
@@ -185,8 +186,8 @@ __device__ __forceinline__ void skinny_prologue(const SkinnyArgs& a, T* xs, floa
         }
     } else if (PRO == PRO_RMSNORM) {
         // forward.hpp:34-56: y = x * rsqrt(mean(x^2) + eps) * w.  8 / Mp warps share a row; each keeps
-        // up to 4 quads per lane in registers between the sum of squares and the scaling.
-        constexpr int CACHE = 4;
+        // up to HELD quads per lane in registers between the sum of squares and the scaling.
+        constexpr int CACHE = HELD;
         const int wpr = kSkinnyWarps / Mp;                      // warps per row
         const int m = warp / wpr, part = warp % wpr;
         const int quads = K / 4, qper = (quads + wpr - 1) / wpr;
@@ -807,7 +808,8 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
             __syncwarp();
             if constexpr (PRO == PRO_SCALED) fold_load(a, warp, lane, sums);
         } else {
-            skinny_prologue<T, PRO>(a, xs, part_ss, Mp, warp, lane);
+            // (queries from a latent of up to 1536 columns, eight rows: one trip to memory)
+            skinny_prologue<T, PRO, false, EPI == EPI_PAIRROT ? 12 : 4>(a, xs, part_ss, Mp, warp, lane);
         }
         const int rows = pro_rows16(PRO) ? a.M : Mp;              // rows of X in shared memory
         const T* xrow = xs + size_t(g) * xstride + t4 * 16;

@@ -417,7 +417,7 @@ int gqa_build(b200p_session* s) {
     b200p_decode_args a{};
     a.D = D; a.N = s->max_seq; a.nQHeads = c.n_heads; a.nKVHeads = c.n_kv_heads; a.stride_kv = s->max_seq; a.batch = s->batch; a.dtype = s->dtype;
     size_t need = 0;
-    for (int n = 1; n <= s->max_seq; n = n < 128 ? 128 : n * 2) {       // the split plan depends on N: take the largest need
+    for (int n = 128;; n += 128) {                                      // the split plan depends on N: take the largest need
         a.N = n < s->max_seq ? n : s->max_seq;
         const size_t b = b200p_attn_decode_workspace_bytes(&a);
         need = b > need ? b : need;

@@ -13,7 +13,7 @@
 //   research/flash-attention-mi300x/kernels/fa_dpp.hip:167-313
 // whose launch takes (seq_len, n_heads, scale).
 //
-// Tiling is the reference's: Br = 16 query rows per CTA (two per warp),
+// Tiling is the reference's: Br = 16 query rows per CTA (four or two per warp),
 // Bc = 64 keys per tile.  A 64-key score row is held by ONE 32-lane warp as an
 // adjacent pair per lane (keys 2l, 2l+1), which is exactly the shape the pair
 // overloads of wave64.cuh reduce; O stays in registers (D/32 dims per lane)
@@ -49,73 +49,80 @@ template <> __device__ __forceinline__ float exp_for<float>(float x)         { r
 template <> __device__ __forceinline__ float exp_for<__half>(float x)        { return __expf(x); }
 template <> __device__ __forceinline__ float exp_for<__nv_bfloat16>(float x) { return __expf(x); }
 
-// What bounds this kernel is shared memory: a warp with one row reads the whole K and V tile for it, and q again for every
-// lane (40 KB per row and tile).  Here two rows share each read, and every lane reads its own two key rows at the same
-// 16-byte chunk, so q is a broadcast; the keys lie 16 bytes further apart than their size, odd keys behind the even ones, and
-// the eight lanes of a shared-memory phase hit eight different bank groups.  (Four rows per warp read less but leave too
-// few warps: within 10 % at 8 heads x 512 keys either way.)  Before and after: 8 heads of 64, 512 keys, fp32, step 1
-// 57.7 -> 38.0 us, step 2 54.6 -> 34.6 (its copies were bulk copies behind an mbarrier and an abort word to clear); 12 heads, 333 keys,
-// fp32, which went to the one-row kernels: step 1 110.6 -> 29.2; 24 heads of 128, 1024 keys, fp16: 675 -> 505.
+// What bounds this kernel is shared memory: a warp reads the whole K and V tile for its rows, and q and the weights as broadcasts.
+// Four rows of a warp share each read (12 wavefronts for 32 FMAs; two rows 20, one row 40 KB per row and tile), and so that
+// there are still eight warps for 16 rows, they are two groups that take every other tile; the second group's maxima, sums and O join
+// the first's at the end.  (fp32 heads of 128: one group of two rows a warp, two tiles would
+// leave no second CTA.)  Every lane reads
+// its own two key rows at the same 16-byte chunk, so q is a broadcast; the keys lie 16 bytes further apart than their size, odd keys
+// behind the even ones, and the eight lanes of a shared-memory phase hit eight different bank groups.  Against one group of two
+// rows a warp, graph replays, step 1 / step 2: 8 heads of 64, 512 keys, fp32 37.9 / 34.5 -> 29.4 / 28.2 us, fp16 30.4 / 30.0 -> 26.7 / 25.0;
+// 24 heads, 1024 keys, fp32 352 / 327 -> 300 / 279; fp16, heads of 128, 498 / 505 -> 438 / 479.
 // Lengths need not be multiples of the tiles: keys past the end get no weight, rows past the end are not stored.
-constexpr int kRowsPerWarp = 2, kStepThreads = kBr / kRowsPerWarp * 32;
+constexpr int kStepWarps = 8, kStepThreads = kStepWarps * 32;
 template <typename T, int D> struct StepTile {
+    static constexpr int MAX_G = D * int(sizeof(T)) <= 256 ? 2 : 1;       // groups of warps (below) whose tiles fit an SM
     static constexpr int ROW = D * int(sizeof(T));                         // bytes of a key
     static constexpr int KROW = ROW + 16;                                  // between two slots of K
     static constexpr int K_BYTES = kBc * KROW, V_BYTES = kBc * ROW;
 };
 
-template <typename T, int D, int STEP>
-__global__ void __launch_bounds__(kStepThreads)
+template <typename T, int D, int STEP, int G, int VB>
+__global__ void __launch_bounds__(kStepThreads, 2)
 fa_step_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V, T* __restrict__ O,
                int seq_q, int seq_k, int heads, float scale, float m_first) {
     using Sh = StepTile<T, D>;
     constexpr int DPL = D / 32;                           // output dims per lane
-    constexpr int NB = STEP == 2 ? 2 : 1;                 // tile buffers
-    constexpr int R = kRowsPerWarp;
+    constexpr int NB = STEP == 2 ? 2 : 1;                                  // buffers of K (VB of V)
+    constexpr int R = 2 * G, WG = kStepWarps / G;                         // rows per warp, warps of a group
     extern __shared__ __align__(128) unsigned char smem[];
-    unsigned char* Kt = smem;                                              // [NB][kBc slots][KROW]: key k in slot (k % 2) * 32 + k / 2
-    unsigned char* Vt = smem + NB * Sh::K_BYTES;                           // [NB][kBc][D]
-    float* prow = reinterpret_cast<float*>(Vt + NB * Sh::V_BYTES);         // [Br][Bc]
-    float* qs = prow + kBr * kBc;                                          // [Br][D]
+    unsigned char* Kt = smem;                                              // [NB][G][kBc slots][KROW]: key k in slot (k % 2) * 32 + k / 2
+    unsigned char* Vt = smem + NB * G * Sh::K_BYTES;                       // [VB][G][kBc][D]
+    float* prow = reinterpret_cast<float*>(Vt + VB * G * Sh::V_BYTES);     // [G][Br][Bc]
+    float* qs = prow + G * kBr * kBc;                                      // [Br][D]
 
     // blockIdx.x = batch * heads * (seq_q/Br) + head * (seq_q/Br) + qblk   (fa_naive.hip:70-71)
     const int qblocks = (seq_q + kBr - 1) / kBr;
     const int qblk = blockIdx.x % qblocks;
     const int bh = blockIdx.x / qblocks;                                   // batch * heads + head
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int row0 = qblk * kBr + warp * R;                                // this warp's first query row
+    const int wrow = warp % WG * R, grp = warp / WG;                       // this warp's first row of the block, its group
+    const int row0 = qblk * kBr + wrow;                                    // this warp's first query row
     const T* Kb = K + size_t(bh) * seq_k * D;
     const T* Vb = V + size_t(bh) * seq_k * D;
     const int ntiles = (seq_k + kBc - 1) / kBc;
 
-    float* q = qs + warp * R * D;
+    float* q = qs + wrow * D;
     #pragma unroll
-    for (int r = 0; r < R; ++r)
+    for (int r = grp; r < R; r += G)                                       // (read behind the first tile's barrier)
         for (int d = lane; d < D; d += 32) q[r * D + d] = row0 + r < seq_q ? to_float(Q[(size_t(bh) * seq_q + row0 + r) * D + d]) : 0.f;
-    __syncwarp();
-    // tile j into buffer j & 1, 16 bytes per thread per step: asynchronous copies (step 2), or through registers
-    auto copy_tile = [&](int j) {
+    // K, V or both of tiles j * G .. into their buffers, 16 bytes per thread per step: asynchronous copies (step 2), or through registers
+    auto copy = [&](int j, bool of_k, bool of_v) {
         constexpr int CPR = Sh::ROW / 16;                                 // chunks per key
-        const int nb = STEP == 2 ? (j & 1) : 0, n = min(kBc, seq_k - j * kBc);
-        const uint4* ks = reinterpret_cast<const uint4*>(Kb + size_t(j) * kBc * D);
-        const uint4* vs = reinterpret_cast<const uint4*>(Vb + size_t(j) * kBc * D);
-        unsigned char* kd = Kt + nb * Sh::K_BYTES;
-        unsigned char* vd = Vt + nb * Sh::V_BYTES;
-        for (int i = threadIdx.x; i < n * CPR; i += kStepThreads) {
-            const int k = i / CPR, c = i % CPR;
-            unsigned char* kslot = kd + ((k & 1) * 32 + (k >> 1)) * Sh::KROW + c * 16;
-            if (STEP == 2) {
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dme::smem_addr(kslot)), "l"(ks + i) : "memory");
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dme::smem_addr(vd + i * 16)), "l"(vs + i) : "memory");
-            } else {
-                *reinterpret_cast<uint4*>(kslot) = ks[i];
-                reinterpret_cast<uint4*>(vd)[i] = vs[i];
+        #pragma unroll
+        for (int t = 0; t < G; ++t) {
+            const int k0 = (j * G + t) * kBc, n = min(kBc, seq_k - k0);
+            const uint4* ks = reinterpret_cast<const uint4*>(Kb + size_t(k0) * D);
+            const uint4* vs = reinterpret_cast<const uint4*>(Vb + size_t(k0) * D);
+            unsigned char* kd = Kt + (j % NB * G + t) * Sh::K_BYTES;
+            unsigned char* vd = Vt + (j % VB * G + t) * Sh::V_BYTES;
+            for (int i = threadIdx.x; i < n * CPR; i += kStepThreads) {
+                const int k = i / CPR, c = i % CPR;
+                unsigned char* kslot = kd + ((k & 1) * 32 + (k >> 1)) * Sh::KROW + c * 16;
+                if (STEP == 2) {
+                    if (of_k) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dme::smem_addr(kslot)), "l"(ks + i) : "memory");
+                    if (of_v) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dme::smem_addr(vd + i * 16)), "l"(vs + i) : "memory");
+                } else {
+                    *reinterpret_cast<uint4*>(kslot) = ks[i];
+                    reinterpret_cast<uint4*>(vd)[i] = vs[i];
+                }
             }
         }
         if (STEP == 2) asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (STEP == 2) copy_tile(0);
+    if (STEP == 2) copy(0, true, VB == 2);
 
+    float* const pw = prow + (grp * kBr + wrow) * kBc;                      // this warp's weights
     float m[R], l[R], o[R][DPL];
     #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -124,17 +131,28 @@ fa_step_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __rest
         for (int i = 0; i < DPL; ++i) o[r][i] = 0.f;
     }
 
-    for (int j = 0; j < ntiles; ++j) {
-        const int buf = STEP == 2 ? (j & 1) : 0, live = min(kBc, seq_k - j * kBc);
-        const unsigned char* Kc = Kt + buf * Sh::K_BYTES;
-        unsigned char* Vc = Vt + buf * Sh::V_BYTES;
-        if (STEP == 2) {                                                   // prefetch tile j + 1, wait for tile j
-            if (j + 1 < ntiles) { copy_tile(j + 1); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+    const int steps = (ntiles + G - 1) / G;
+    for (int j = 0; j < steps; ++j) {
+        const int buf = STEP == 2 ? (j & 1) : 0, live = min(kBc, seq_k - (j * G + grp) * kBc);
+        const unsigned char* Kc = Kt + (buf * G + grp) * Sh::K_BYTES;
+        const unsigned char* Vc = Vt + (j % VB * G + grp) * Sh::V_BYTES;
+        // no weight times whatever was there must be nothing
+        auto clear_tail = [&] {
+            if (j + 1 < steps || seq_k % kBc == 0) return;
+            uint4* Vl = reinterpret_cast<uint4*>(Vt + (j % VB * G + (ntiles - 1) % G) * Sh::V_BYTES);
+            for (int i = seq_k % kBc * (Sh::ROW / 16) + threadIdx.x; i < kBc * (Sh::ROW / 16); i += kStepThreads) Vl[i] = make_uint4(0u, 0u, 0u, 0u);
+        };
+        if (STEP == 2 && VB == 1) {                                        // V travels under the scores, the next K under the whole step
+            copy(j, false, true);
+            if (j + 1 < steps) { copy(j + 1, true, false); asm volatile("cp.async.wait_group 2;" ::: "memory"); }
+            else asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else if (STEP == 2) {                                            // prefetch the next tiles, wait for these
+            if (j + 1 < steps) { copy(j + 1, true, true); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
             else asm volatile("cp.async.wait_group 0;" ::: "memory");
-        } else copy_tile(j);
-        if (live < kBc)                                                    // no weight times whatever was there must be nothing
-            for (int i = live * (Sh::ROW / 16) + threadIdx.x; i < kBc * (Sh::ROW / 16); i += kStepThreads) reinterpret_cast<uint4*>(Vc)[i] = make_uint4(0u, 0u, 0u, 0u);
+            clear_tail();
+        } else { copy(j, true, true); clear_tail(); }
         __syncthreads();
+        if (G == 1 || live > 0) {                                          // (the last step may have no tile for this group)
         // S[row][2l], S[row][2l+1]
         float s0[R], s1[R];
         #pragma unroll
@@ -173,15 +191,23 @@ fa_step_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __rest
             m[r] = m_new;
             #pragma unroll
             for (int i = 0; i < DPL; ++i) o[r][i] *= resc;
-            *reinterpret_cast<float2*>(&prow[(warp * R + r) * kBc + 2 * lane]) = make_float2(p0, p1);
+            *reinterpret_cast<float2*>(&pw[r * kBc + 2 * lane]) = make_float2(p0, p1);
         }
         __syncwarp();
+        }
+        if (STEP == 2 && VB == 1) {
+            if (j + 1 < steps) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 0;" ::: "memory");
+            clear_tail();
+            __syncthreads();
+        }
+        if (G == 1 || live > 0) {
         // O[row][d] += sum_k P[row][k] * V[k][d]
         #pragma unroll 2
         for (int k = 0; k < kBc; k += 4) {
             float4 p4[R];
             #pragma unroll
-            for (int r = 0; r < R; ++r) p4[r] = *reinterpret_cast<const float4*>(&prow[(warp * R + r) * kBc + k]);      // broadcast reads
+            for (int r = 0; r < R; ++r) p4[r] = *reinterpret_cast<const float4*>(&pw[r * kBc + k]);      // broadcast reads
             #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
                 float v[DPL];
@@ -195,7 +221,29 @@ fa_step_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __rest
                 }
             }
         }
+        }
         __syncthreads();                                  // tile buffers and prow are reused next iteration
+    }
+    if (G == 2) {                                         // the second group's part of the rows joins the first's
+        float* part = reinterpret_cast<float*>(Kt) + (warp % WG) * R * (D + 2);       // [R][D] sums, [R] m, [R] l
+        static_assert(WG * R * (D + 2) * int(sizeof(float)) <= Sh::K_BYTES);
+        if (grp == 1) {
+            #pragma unroll
+            for (int r = 0; r < R; ++r) {
+                #pragma unroll
+                for (int i = 0; i < DPL; ++i) part[r * D + lane * DPL + i] = o[r][i];
+                if (lane == 0) { part[R * D + r] = m[r]; part[R * D + R + r] = l[r]; }
+            }
+        }
+        __syncthreads();
+        if (grp == 1) return;
+        #pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float mo = part[R * D + r], m_new = fmaxf(m[r], mo), a = exp_for<T>(m[r] - m_new), b = exp_for<T>(mo - m_new);
+            l[r] = a * l[r] + b * part[R * D + R + r];
+            #pragma unroll
+            for (int i = 0; i < DPL; ++i) o[r][i] = a * o[r][i] + b * part[r * D + lane * DPL + i];
+        }
     }
     #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -336,13 +384,20 @@ template <typename T, int D, int STEP>
 int launch_step(const void* Q, const void* K, const void* V, void* O, int batch, int heads, int seq_q, int seq_k,
                 float scale, float m_first, cudaStream_t st) {
     using Sh = StepTile<T, D>;
-    const size_t smem = size_t(STEP == 2 ? 2 : 1) * (Sh::K_BYTES + Sh::V_BYTES) + (kBr * kBc + kBr * D) * sizeof(float);
-    auto kern = fa_step_kernel<T, D, STEP>;
+    // two groups of warps wherever there are two tiles for them (one tile, 1 head of 64, fp16: 4.4 us with one, 5.2 with two)
+    const int G = seq_k > kBc ? Sh::MAX_G : 1;
+    const unsigned grid = unsigned(batch) * heads * ((seq_q + kBr - 1) / kBr);
+    // Step 2's fp32 tiles with one buffer of V leave room for a second CTA on an SM, if there is one (8 heads of 64, 512 keys: 36.0 us with two
+    // buffers, 28.3 with one; of 128: 68.9 and 58.9, but 1 head 35.0 and 36.8; fp16, 8 heads of 128: 47.2 and 50.1)
+    constexpr int MOST = STEP == 2 ? 2 : 1;
+    const int VB = MOST == 2 && sizeof(T) == 4 && grid > unsigned(sm_count()) ? 1 : MOST;
+    const size_t smem = G * (size_t(MOST) * Sh::K_BYTES + size_t(VB) * Sh::V_BYTES) + (G * kBr * kBc + kBr * D) * sizeof(float);
+    auto kern = G == 2 ? fa_step_kernel<T, D, STEP, Sh::MAX_G, MOST> : fa_step_kernel<T, D, STEP, 1, MOST>;
+    if constexpr (sizeof(T) == 4) if (VB == 1) kern = G == 2 ? fa_step_kernel<T, D, STEP, Sh::MAX_G, 1> : fa_step_kernel<T, D, STEP, 1, 1>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return int(e);
     }
-    const unsigned grid = unsigned(batch) * heads * ((seq_q + kBr - 1) / kBr);
     kern<<<grid, kStepThreads, smem, st>>>(static_cast<const T*>(Q), static_cast<const T*>(K), static_cast<const T*>(V),
                                        static_cast<T*>(O), seq_q, seq_k, heads, scale, m_first);
     return launched();
@@ -410,9 +465,6 @@ extern "C" int b200p_fa_step(int step, int dtype, const void* Q, const void* K, 
         if (dtype != B200P_F32 || seq_q != seq_k) return B200P_E_LENGTH;
         if ((long long)batch * heads > 65535) return B200P_E_RANGE;      // as in b200p_fa_rows_f32, the other entry for such lengths
         m_first = -3.402823466e+38f;
-        // Two buffers of 128 fp32 columns leave an SM one CTA: 8 heads, 333 keys, step 1 47.6 us, step 2 52.8; 2 x 12 heads 92.1 and
-        // 104.0.  There step 2 runs step 1 (same bits).  With 64 columns step 2 is the faster one: 28.8 and 26.3 us.
-        if (step == 2 && D == 128) step = 1;
     }
     switch (dtype) {
         case B200P_F16:  return launch_step_d<__half>(step, D, Q, K, V, O, batch, heads, seq_q, seq_k, scale, m_first, st);

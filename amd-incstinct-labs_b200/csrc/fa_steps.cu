@@ -68,7 +68,7 @@ template <typename T, int D> struct StepTile {
 };
 
 template <typename T, int D, int STEP, int G, int VB>
-__global__ void __launch_bounds__(kStepThreads, 2)
+__global__ void __launch_bounds__(kStepThreads, D * sizeof(T) > 256 && STEP != 0 ? 1 : 2)      // (fp32 heads of 128, steps 1 and 2, 8 heads, 512 keys: 64.7 and 60.6 us with 2, 62.8 and 58.9 with 1)
 fa_step_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V, T* __restrict__ O,
                int seq_q, int seq_k, int heads, float scale, float m_first) {
     using Sh = StepTile<T, D>;

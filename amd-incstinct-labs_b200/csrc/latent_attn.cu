@@ -165,25 +165,44 @@ __global__ void __launch_bounds__(kStepThreads) latent_absorb_kernel(const Laten
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, M = a.batch * a.Tn;
     if (int(blockIdx.y) == d.heads) {
         if (blockIdx.x != 0) return;
+        // the position (set by launches that have completed before a step's first kernel, an ordinary launch, starts) and the weights,
+        // ahead of the wait; up to HELD quads of a row per lane between its sum of squares and the scaling
+        constexpr int HELD = 4;
+        const T16* w = static_cast<const T16*>(a.kv_norm);
+        const int pos0 = first_pos(a);
+        uint2 wv[HELD];
+        #pragma unroll
+        for (int i = 0; i < HELD; ++i) {
+            wv[i] = make_uint2(0u, 0u);
+            if (lane + 32 * i < d.rank / 4) wv[i] = *reinterpret_cast<const uint2*>(w + 4 * (lane + 32 * i));
+        }
         griddep_wait();
         for (int m = warp; m < M; m += kStepWarps) {
             const float* p = a.proj + size_t(m) * d.proj_row() + d.qrank;
-            const T16* w = static_cast<const T16*>(a.kv_norm);
-            const int pos = first_pos(a) + m % a.Tn;
+            const int pos = pos0 + m % a.Tn;
             T16* row = static_cast<T16*>(a.cache) + (size_t(m / a.Tn) * a.max_seq + pos) * d.cache_row();
+            float4 held[HELD];
             float ss = 0.f;
-            for (int q = lane; q < d.rank / 4; q += 32) {
+            #pragma unroll
+            for (int i = 0; i < HELD; ++i) {
+                held[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (lane + 32 * i < d.rank / 4) held[i] = *reinterpret_cast<const float4*>(p + 4 * (lane + 32 * i));
+            }
+            #pragma unroll
+            for (int i = 0; i < HELD; ++i) ss += held[i].x * held[i].x + held[i].y * held[i].y + held[i].z * held[i].z + held[i].w * held[i].w;
+            for (int q = lane + 32 * HELD; q < d.rank / 4; q += 32) {
                 const float4 v = *reinterpret_cast<const float4*>(p + 4 * q);
                 ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
             }
             const float inv = rsqrtf(wave::dpp::reduce_sum(ss) / a.kv_rank + a.eps);
-            for (int q = lane; q < d.rank / 4; q += 32) {
-                const float4 v = *reinterpret_cast<const float4*>(p + 4 * q);
-                const uint2 wv = *reinterpret_cast<const uint2*>(w + 4 * q);
-                const T16* g = reinterpret_cast<const T16*>(&wv);
+            auto put = [&](int q, const float4& v, const uint2& wq) {
+                const T16* g = reinterpret_cast<const T16*>(&wq);
                 *reinterpret_cast<uint2*>(row + 4 * q) = make_uint2(pack2<T16>(v.x * inv * to_float(g[0]), v.y * inv * to_float(g[1])),
                                                                     pack2<T16>(v.z * inv * to_float(g[2]), v.w * inv * to_float(g[3])));
-            }
+            };
+            #pragma unroll
+            for (int i = 0; i < HELD; ++i) if (lane + 32 * i < d.rank / 4) put(lane + 32 * i, held[i], wv[i]);
+            for (int q = lane + 32 * HELD; q < d.rank / 4; q += 32) put(q, *reinterpret_cast<const float4*>(p + 4 * q), *reinterpret_cast<const uint2*>(w + 4 * q));
             const float* k = p + d.rank;
             for (int i = lane; i < d.rot / 2; i += 32) {
                 const int u = 16 * (i / 8) + i % 8;
@@ -474,13 +493,13 @@ __global__ void __launch_bounds__(kStepThreads) latent_merge_kernel(const Latent
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, h = blockIdx.x % d.heads;
     const size_t row = blockIdx.x;
     const int c = (blockIdx.y * 32 + lane) * 4;
-    griddep_wait();
     int N, per;
-    step_extent(a, splits, N, per);
+    step_extent(a, splits, N, per);                                 // (the position is older than the step: read ahead of the wait)
     const int used = (N + per - 1) / per;                           // splits with keys
+    const float sink = a.sink ? a.sink[h] * 1.4426950408889634f : kNegBig;
+    griddep_wait();
     if (warp == 0) {
         constexpr int PER = kMaxSplits / 32;
-        const float sink = a.sink ? a.sink[h] * 1.4426950408889634f : kNegBig;
         float2 ml[PER];
         float top = sink;
         #pragma unroll

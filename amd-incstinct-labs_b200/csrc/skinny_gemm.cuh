@@ -207,6 +207,7 @@ __device__ __forceinline__ void skinny_prologue(const SkinnyArgs& a, T* xs, floa
         if (m < a.M) {
             #pragma unroll
             for (int it = 0; it < CACHE; ++it) {
+                if (it >= 4 && q0 + 32 * it >= q1) break;
                 const int q = q0 + lane + 32 * it;
                 if (q < q1) {
                     cx[it] = ldx(q);
@@ -247,6 +248,7 @@ __device__ __forceinline__ void skinny_prologue(const SkinnyArgs& a, T* xs, floa
         if (m < a.M) {
             #pragma unroll
             for (int it = 0; it < CACHE; ++it) {
+                if (it >= 4 && q0 + 32 * it >= q1) break;
                 const int q = q0 + lane + 32 * it;
                 if (q < q1) put(q, cx[it], cw[it]);
             }
@@ -770,7 +772,6 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
                     const int c0 = sl * slab, cols = min(slab, K - c0);
                     unsigned char* dst = stages + size_t(stage) * stage_bytes;
                     dme::mbar_arrive_expect_tx(&full_bar[stage], uint32_t(16 * cols * 2));
-                    #pragma unroll 2
                     for (int r = 0; r < 16; ++r) {
                         size_t row;
                         if (epi_gated(EPI))    row = r < 8 ? size_t(min(grp * 8 + r, a.N - 1)) : size_t(a.N) + size_t(min(grp * 8 + r - 8, a.N - 1));

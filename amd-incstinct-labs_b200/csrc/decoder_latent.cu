@@ -621,6 +621,7 @@ int latent_build(b200p_session* s, const b200p_model* m) {
         L->cache.push_back(cache);
     }
     s->skinny_max_k = max_k;
+    s->fold_max_k = L->H;
     s->skinny_usable = s->dtype != B200P_F32;
     if (s->skinny_usable && s->batch <= kSkinnyMaxM) s->fold_first = s->final_norm;      // only the head's norm is folded
     if (cudaError_t e = s->alloc(&L->kv, size_t(s->batch) * s->max_seq * L->max_kv * esz)) return int(e);

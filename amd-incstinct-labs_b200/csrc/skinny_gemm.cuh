@@ -927,6 +927,22 @@ inline bool skinny_rows_fit(int M, int K) {
     return M <= kSkinnyMaxM && size_t(M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16) * size_t(K + kSkinnyXPad) * 2 <= 190 * 1024;
 }
 
+// The ring of the streaming kernel beside M rows of K columns of X: columns and bytes of a stage, stages (two at least, or it does not run).
+struct SkinnyRing { int slab_cols, stage_bytes, nstages, x_bytes; };
+inline SkinnyRing skinny_ring(int M, int K) {
+    const int Mp = M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
+    SkinnyRing r{};
+    r.slab_cols = kSkinnySlab;                                          // measured: 0.67 ms per token at 2048, 0.72 at 1024, 0.73 at 4096
+    r.x_bytes = int((size_t(Mp) * (K + kSkinnyXPad) * 2 + 127) / 128 * 128);
+    const int room = 223488 - (M > 8 ? 8192 : 0) - r.x_bytes;
+    // half a stage where X leaves room for one whole stage only (16 rows of 3072)
+    if (K > r.slab_cols && room / (16 * (r.slab_cols * 2 + 16)) == 1) r.slab_cols /= 2;
+    r.stage_bytes = 16 * ((K < r.slab_cols ? K : r.slab_cols) * 2 + 16);
+    r.nstages = room / r.stage_bytes;
+    if (r.nstages > 8) r.nstages = 8;
+    return r;
+}
+
 // Launch of shapes in skinny_domain (skinny_tc.cuh, which chooses between these kernels and its own); B200P_E_RANGE: they
 // do not fit these kernels either.  *parts: EPI_ADD_FOLD's number of partial sums.  The folded forms have no register kernel.
 template <typename T, int PRO, int EPI, int MH>
@@ -939,14 +955,9 @@ int launch_skinny_mh(const SkinnyArgs& a, cudaStream_t st, int* parts = nullptr)
     const bool pdl = tuning(KNOB_RUNTIME_PDL, 1) != 0;
     if (tuning(KNOB_RUNTIME_SKINNY, 2) == 2 && aligned(a.W, 16)) {
         // W staged through shared memory by a producer thread (skinny_stream_kernel), one CTA per SM
-        int slab_cols = kSkinnySlab;                                     // measured: 0.67 ms per token at 2048, 0.72 at 1024, 0.73 at 4096
-        const int x_bytes = int((smem + 127) / 128 * 128);
-        // half a stage where X leaves room for one whole stage only (16 rows of 3072)
-        if (a.K > slab_cols && (223488 - 8192 * (MH - 1) - x_bytes) / (16 * (slab_cols * 2 + 16)) == 1) slab_cols /= 2;
-        const int slab = a.K < slab_cols ? a.K : slab_cols;
-        const int stage_bytes = 16 * (slab * 2 + 16);
-        int nstages = (223488 - 8192 * (MH - 1) - x_bytes) / stage_bytes;
-        if (nstages > 8) nstages = 8;
+        const SkinnyRing ring = skinny_ring(a.M, a.K);
+        const int slab_cols = ring.slab_cols, x_bytes = ring.x_bytes, stage_bytes = ring.stage_bytes;
+        int nstages = ring.nstages;
         // A few more row groups than SMs (the decode step's Q/K/V: 160 on 148), each one stage long: with one CTA per
         // SM a dozen CTAs would take two groups one after the other and the whole grid would wait for them.  One CTA
         // per group with a single stage instead: two of them fit an SM and run side by side.

@@ -583,6 +583,15 @@ inline bool skinny_split(int M, int K, size_t bytes, bool own_abort_word) {
     return size_t(Mp) * K * 2 > 96 * 1024 && (own_abort_word || bytes > size_t(M > 8 ? 20 : 64) << 20);
 }
 
+// Whether M rows of K columns run on a kernel that has the folded forms (this file's or the streaming one: the register kernel has
+// none), for a caller with an abort word of its own.  Holds for fewer columns too where it holds for K.
+inline bool skinny_folds(int M, int K) {
+    const int kind = tuning(KNOB_RUNTIME_SKINNY, 2);
+    if (M > kSkinnyMaxM || kind < 2) return false;
+    if ((kind == 3 || skinny_split(M, K, 0, true)) && skinny_tc_fits(M, K)) return true;
+    return kind == 2 && skinny_rows_fit(M, K) && skinny_ring(M, K).nstages >= 2;
+}
+
 // B200P_E_RANGE: the shape is outside the kernel's domain (nothing was launched).
 template <typename T, int PRO, int EPI, int NB>
 int launch_skinny_tc(const SkinnyArgs& a, cudaStream_t st, int* parts = nullptr) {

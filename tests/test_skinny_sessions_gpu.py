@@ -42,6 +42,14 @@ def test_rows_too_long_for_every_allowed_split_take_the_gemm(b200p, torch_cuda):
     steps(b200p, torch_cuda, llama(4, 2, 64, ffn=12304, hidden=256), "bf16", False, 8)
 
 
+# rows that fit the register kernel, but neither two stages of the streaming one beside them nor one CTA of the cluster kernel: the
+# down projection's, with 16 and with 8 sequences, and the O projection's
+@pytest.mark.parametrize("heads,kv,ffn,batch", [(4, 2, 5632, 16), (4, 2, 9856, 8), (88, 8, 512, 16)])
+def test_rows_that_no_kernel_with_a_folded_norm_takes(b200p, torch_cuda, heads, kv, ffn, batch):
+    b200p.set_tuning("skinny_cluster", 1)
+    steps(b200p, torch_cuda, llama(heads, kv, 64, ffn=ffn, hidden=256), "bf16", False, batch)
+
+
 # heads whose rows fill the 128-row tiles and not, one head a tile and two, biases, one and two fragments of rows
 @pytest.mark.parametrize("cluster", [0, 1, 3, 8])
 @pytest.mark.parametrize("heads,kv,D,kind,bias,batch", [(8, 2, 64, "bf16", False, 1), (3, 3, 64, "f16", True, 3), (4, 1, 128, "bf16", True, 9), (5, 5, 64, "bf16", True, 16),

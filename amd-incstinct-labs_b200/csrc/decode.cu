@@ -74,8 +74,8 @@ struct DecodeParams {
     // to finish merges that unit's splits and writes o; tickets[batch * nKVH] count arrivals
     // and reset themselves.  Null: the partials are left for a separate combine launch.
     void* fused_o; unsigned int* tickets; long long o_batch_stride;
-    int pdl;                      // host only: launch the tensor-core kernel as a programmatic dependent
-    int cluster;                  // fused combine with all splits of a unit in one thread-block cluster: they meet in shared memory
+    int pdl;                      // the tensor-core kernel is launched as a programmatic dependent
+    int cluster;                  // host only: fused combine with all splits of a unit in one thread-block cluster (decode_mma_kernel's CLUSTER)
     int o_pairs;                  // fused output: rows start on 4 bytes, so two 16-bit results go out as one word
 };
 
@@ -365,7 +365,10 @@ __device__ __forceinline__ float2 load_cluster(uint32_t smem, uint32_t cta) {
     asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
     return v;
 }
-template <typename T, int D>
+// CLUSTER: all splits of a unit are one thread-block cluster and meet in shared memory.  An instantiation of its own: with that merge behind
+// a branch of the other, calls without a cluster took longer, the same registers or not (heads of 64: 8 of 8, 5 sequences, 2100 keys 14.7 -> 15.7 us,
+// 16 sequences, 1025 keys 20.7 -> 21.7; 32 / 4, 16 sequences, 900 keys 9.0 -> 9.9; apart 14.7, 20.7 and 9.0).
+template <typename T, int D, bool CLUSTER>
 __global__ void __launch_bounds__(kDecodeThreads, 1)
 decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV) {
     using Sh = DecodeShape<D>;
@@ -564,7 +567,7 @@ decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap mapK
                 L += f * ml.y;
                 O0 += f * ov.x; O1 += f * ov.y;
             }
-            if (p.fused_o && p.splits == 1) {
+            if (!CLUSTER && p.fused_o && p.splits == 1) {
                 // the only split of its unit: this is the result, no partials and no merge
                 T* dst = static_cast<T*>(p.fused_o) + size_t(b) * p.o_batch_stride + (size_t(kvh) * p.group + hh) * D + d;
                 const float r0 = L > 0.f ? O0 / L : O0, r1 = L > 0.f ? O1 / L : O1;
@@ -572,7 +575,7 @@ decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap mapK
                 else { dst[0] = from_float<T>(r0); dst[1] = from_float<T>(r1); }
                 continue;
             }
-            if (p.cluster) {
+            if (CLUSTER) {
                 *reinterpret_cast<float2*>(&cl_o[hh * D + d]) = make_float2(O0, O1);
                 if (d == 0) *reinterpret_cast<float2*>(&cl_ml[hh * 2]) = make_float2(M, L);
                 continue;
@@ -582,7 +585,7 @@ decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap mapK
             if (d == 0) { p.part_ml[row * 2] = M; p.part_ml[row * 2 + 1] = L; }
         }
     }
-    if (p.cluster) {
+    if constexpr (CLUSTER) {
         // ---- the unit's splits are the CTAs of this cluster: each merges its share of the columns from all of them through
         // distributed shared memory (the same sums as below, without partials in global memory and a ticket) ----
         __syncwarp();
@@ -929,13 +932,13 @@ int launch_decode_mma(const DecodeParams& p, const b200p_decode_args* a, cudaStr
     cudaError_t e = make_tensor_map(&mk, dt, 4, p.K, dims, strides, box, Swizzle::B128);
     if (e == cudaSuccess) e = make_tensor_map(&mv, dt, 4, p.V, dims, strides, box, Swizzle::B128);
     if (e != cudaSuccess) return int(e);
-    auto kern = decode_mma_kernel<T, D>;
-    static bool attr_set[64] = {};
+    auto kern = p.cluster ? decode_mma_kernel<T, D, true> : decode_mma_kernel<T, D, false>;
+    static bool attr_set[2][64] = {};                   // [CLUSTER][device]
     int dev = 0; cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+    if (dev >= 0 && dev < 64 && !attr_set[p.cluster][dev]) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::SMEM_BYTES);
         if (e != cudaSuccess) return int(e);
-        attr_set[dev] = true;
+        attr_set[p.cluster][dev] = true;
     }
     dim3 grid(p.splits, p.nKVH, p.batch);
     if (p.pdl || p.cluster) {

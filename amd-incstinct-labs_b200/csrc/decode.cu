@@ -1008,7 +1008,9 @@ int run_decode(const b200p_decode_args* a, const void* q, const void* K, const v
     DecodePlan pl = plan_decode(a->D, a->N, a->nQHeads, a->nKVHeads, a->batch);
     // A decode step's launch, a programmatic dependent, has most of its tiles before its wait: 22 layers, without clusters and with, 2 sequences,
     // 577 keys 0.564 and 0.570 ms, 941 keys the same, 1541 keys 0.617 and 0.585; 8 / 16 sequences, 1141 keys 0.725 / 1.15 and 0.629 / 0.989.
-    if (pl.cluster && (!fused || (prepared && a->N <= 1024) || ws_bytes < pl.ws_bytes)) pl = plan_decode(a->D, a->N, a->nQHeads, a->nKVHeads, a->batch, false);
+    // A count read on the device may lie far below the bound, and one tile is no work for a cluster.  32 / 8 heads of 128, bound 1000, without and with:
+    // 1 sequence, 60 / 300 / 1000 keys 6.2 / 8.3 / 10.3 and 8.3 / 8.3 / 8.3 us; bounds above 1024 split either way (1500, 60 keys 10.1 and 8.3).
+    if (pl.cluster && (!fused || ((prepared || n_dev) && a->N <= 1024) || ws_bytes < pl.ws_bytes)) pl = plan_decode(a->D, a->N, a->nQHeads, a->nKVHeads, a->batch, false);
     if (!ws || ws_bytes < pl.ws_bytes || !aligned(ws, 256)) return B200P_E_WORKSPACE;
 
     DecodeParams p{};

@@ -49,6 +49,18 @@ def test_counts_on_the_device(b200p, torch_cuda):
         assert b200p.workspace_status(ws) == 0
 
 
+# bounds on both sides of the one below which a count on the device takes no cluster
+@pytest.mark.parametrize("bound", [513, 1000, 1024, 1025, 2048, 2049])
+@pytest.mark.parametrize("B,H,G,D", [(1, 32, 8, 128), (5, 8, 8, 64)])
+def test_counts_below_the_bound(b200p, torch_cuda, bound, B, H, G, D):
+    torch = torch_cuda
+    q, K, V = case(torch, B, H, G, 2100, D, torch.float16)
+    for n in (1, 60, 128, 300, 512, 513, bound):
+        got = b200p.decode_dyn(q, K, V, torch.tensor([n], dtype=torch.int32, device="cuda"), N=bound)
+        want, limit = expect(torch, q, K, V, n)
+        assert ((got - want).abs() <= limit).all(), n
+
+
 @pytest.mark.parametrize("max_seq,batch", [(1025, 16), (1100, 2), (2047, 8)])
 def test_sessions(b200p, torch_cuda, max_seq, batch):
     """(Their scratch was sized at 1024 keys and every step refused.)"""

@@ -33,7 +33,7 @@ def test_lengths(b200p, torch_cuda, B, H, G, D, N):
         want, bound = expect(torch, q, K, V, N)
         assert ((got - want).abs() <= bound).all()
         small = torch.empty(b200p.decode_workspace(q, K[:, :, :512].contiguous(), 512).numel(), dtype=torch.uint8, device="cuda")
-        if N <= 1024:                                            # scratch of one split: the launch without a cluster
+        if N <= 1024:                                            # scratch of one split
             assert ((b200p.decode(q, K, V, N=N, workspace=small) - want).abs() <= bound).all()
         assert ((b200p.decode_noalloc(q, K, V, N=N) - want).abs() <= bound).all()
 
@@ -47,6 +47,21 @@ def test_counts_on_the_device(b200p, torch_cuda):
         want, bound = expect(torch, q, K, V, n)
         assert ((got - want).abs() <= bound).all(), n
         assert b200p.workspace_status(ws) == 0
+
+
+# one split up to 1024 keys, one per 256 above (few units): what a caller may have sized, whichever form the splits take
+@pytest.mark.parametrize("N,splits", [(700, 1), (1024, 1), (1025, 5), (2000, 8)])
+def test_scratch_of_the_stated_size_is_enough_and_less_is_refused(b200p, torch_cuda, N, splits):
+    torch = torch_cuda
+    q, K, V = case(torch, 1, 32, 32, 2100, 64, torch.float16)
+    ws = b200p.decode_workspace(q, K, N)
+    up = lambda n: -(-n // 256) * 256
+    assert ws.numel() == 256 + up(32 * 4) + up(32 * splits * 8) + 32 * splits * 64 * 4
+    want, bound = expect(torch, q, K, V, N)
+    assert ((b200p.decode(q, K, V, N=N, workspace=ws) - want).abs() <= bound).all()
+    with pytest.raises(b200p.B200PError) as e:
+        b200p.decode(q, K, V, N=N, workspace=ws[:-256])
+    assert e.value.status == -7
 
 
 # bounds on both sides of the one below which a count on the device takes no cluster

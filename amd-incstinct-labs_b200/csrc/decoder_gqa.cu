@@ -464,7 +464,7 @@ extern "C" b200p_session* b200p_session_create(const b200p_model_weights* w, int
         if (!L.Wq || !L.Wk || !L.Wv || !L.Wo || !L.Wgate || !L.Wup || !L.Wdown || !L.norm_attn || !L.norm_mlp) {
             *status = B200P_E_NULL; delete s; return nullptr;
         }
-    if (w->dtype == B200P_BF16 && batch <= kSkinnyMaxM && aligned(s->embed, 8)) s->fold_first = d->layers[0].norm_attn;
+    if (w->dtype == B200P_BF16 && batch <= kSkinnyMaxM && aligned(s->embed, 8)) { s->folds = true; s->fold_first = d->layers[0].norm_attn; }
     int rc = session_common_init(s);
     if (!rc) rc = w->dtype == B200P_F16 ? gqa_build<__half>(s) : gqa_build<__nv_bfloat16>(s);
     if (!rc) rc = int(cudaDeviceSynchronize());

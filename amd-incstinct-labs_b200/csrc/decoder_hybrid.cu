@@ -495,7 +495,7 @@ int hybrid_build(b200p_session* s, const b200p_model* m) {
     if (int rc = s->dtype == B200P_F32 ? build_weights<float>(s, m) : build_weights<__nv_bfloat16>(s, m)) return rc;
     s->skinny_max_k = s->fold_max_k = L->H;               // (sublayer outputs too long for these kernels take the GEMM, and fold_rows)
     s->skinny_usable = s->dtype != B200P_F32;
-    if (s->skinny_usable && s->batch <= kSkinnyMaxM && !L->spec.passes.empty()) s->fold_first = L->w[size_t(L->spec.passes[0].layer)].norm1;
+    if (s->skinny_usable && s->batch <= kSkinnyMaxM && !L->spec.passes.empty()) { s->folds = true; s->fold_first = L->w[size_t(L->spec.passes[0].layer)].norm1; }
     if (cudaError_t e = s->alloc(&s->d_attn_status, 16)) return int(e);
     return int(cudaMemset(s->d_attn_status, 0, 16));
 }

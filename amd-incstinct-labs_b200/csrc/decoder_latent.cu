@@ -623,7 +623,7 @@ int latent_build(b200p_session* s, const b200p_model* m) {
     s->skinny_max_k = max_k;
     s->fold_max_k = L->H;
     s->skinny_usable = s->dtype != B200P_F32;
-    if (s->skinny_usable && s->batch <= kSkinnyMaxM) s->fold_first = s->final_norm;      // only the head's norm is folded
+    s->folds = s->skinny_usable && s->batch <= kSkinnyMaxM;      // the head's norm only: no fold_first
     if (cudaError_t e = s->alloc(&L->kv, size_t(s->batch) * s->max_seq * L->max_kv * esz)) return int(e);
     if (s->dtype == B200P_BF16) {                         // the absorbed attention's queries and partial results
         size_t parts = 0, part_floats = 0, abs = 0;

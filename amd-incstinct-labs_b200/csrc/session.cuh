@@ -108,7 +108,8 @@ struct b200p_session {
     // Decode steps whose norms are folded into the projections around them (SkinnyFold): x * w of the next norm and partial sums
     // of squares.  fold_parts = 0: they do not belong to `hidden`.
     void* fold_x16 = nullptr; float* fold_ss = nullptr;
-    const void* fold_first = nullptr;                    // weights of the first layer's norm; null: the decoder does not fold
+    bool folds = false;                                  // the decoder may fold norms: the two buffers are there
+    const void* fold_first = nullptr;                    // weights of the norm that reads the embeddings; null: it is not folded
     int fold_max_k = 0;                                  // longest row that a folded product without another way out reads
     int fold_parts = 0;
     float* embedded = nullptr;                           // a decoder that reads the embeddings again: a second copy of them (its scratch), or null
@@ -157,7 +158,7 @@ inline bool skinny_ok(const b200p_session* s, int M) {
 
 // Whether the norms of a decode step are folded into the projections around them: bf16 only (SkinnyFold), on the kernels that have the form.
 inline bool fold_ok(const b200p_session* s) {
-    return s->fold_first && s->dtype == B200P_BF16 && skinny_ok(s, s->batch) && skinny_folds(s->batch, s->fold_max_k) && device_status_ptr() != nullptr;
+    return s->folds && s->dtype == B200P_BF16 && skinny_ok(s, s->batch) && skinny_folds(s->batch, s->fold_max_k) && device_status_ptr() != nullptr;
 }
 // The folded form of s->hidden (one row per sequence) for a norm with weights w.
 int fold_rows(b200p_session* s, const void* w, cudaStream_t st);

@@ -67,17 +67,17 @@ template <typename T, int D> struct StepTile {
     static constexpr int K_BYTES = kBc * KROW, V_BYTES = kBc * ROW;
 };
 
-template <typename T, int D, int STEP, int G, int VB>
+// G groups of warps, KB and VB buffers of their tiles of K and V (step 2: 2 and 2, 2 and 1, or 1 and 1; the others: 1 and 1)
+template <typename T, int D, int STEP, int G, int KB, int VB>
 __global__ void __launch_bounds__(kStepThreads, D * sizeof(T) > 256 && STEP != 0 ? 1 : 2)      // (fp32 heads of 128, steps 1 and 2, 8 heads, 512 keys: 64.7 and 60.6 us with 2, 62.8 and 58.9 with 1)
 fa_step_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V, T* __restrict__ O,
                int seq_q, int seq_k, int heads, float scale, float m_first) {
     using Sh = StepTile<T, D>;
     constexpr int DPL = D / 32;                           // output dims per lane
-    constexpr int NB = STEP == 2 ? 2 : 1;                                  // buffers of K (VB of V)
     constexpr int R = 2 * G, WG = kStepWarps / G;                         // rows per warp, warps of a group
     extern __shared__ __align__(128) unsigned char smem[];
-    unsigned char* Kt = smem;                                              // [NB][G][kBc slots][KROW]: key k in slot (k % 2) * 32 + k / 2
-    unsigned char* Vt = smem + NB * G * Sh::K_BYTES;                       // [VB][G][kBc][D]
+    unsigned char* Kt = smem;                                              // [KB][G][kBc slots][KROW]: key k in slot (k % 2) * 32 + k / 2
+    unsigned char* Vt = smem + KB * G * Sh::K_BYTES;                       // [VB][G][kBc][D]
     float* prow = reinterpret_cast<float*>(Vt + VB * G * Sh::V_BYTES);     // [G][Br][Bc]
     float* qs = prow + G * kBr * kBc;                                      // [Br][D]
 
@@ -104,7 +104,7 @@ fa_step_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __rest
             const int k0 = (j * G + t) * kBc, n = min(kBc, seq_k - k0);
             const uint4* ks = reinterpret_cast<const uint4*>(Kb + size_t(k0) * D);
             const uint4* vs = reinterpret_cast<const uint4*>(Vb + size_t(k0) * D);
-            unsigned char* kd = Kt + (j % NB * G + t) * Sh::K_BYTES;
+            unsigned char* kd = Kt + (j % KB * G + t) * Sh::K_BYTES;
             unsigned char* vd = Vt + (j % VB * G + t) * Sh::V_BYTES;
             for (int i = threadIdx.x; i < n * CPR; i += kStepThreads) {
                 const int k = i / CPR, c = i % CPR;
@@ -120,7 +120,7 @@ fa_step_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __rest
         }
         if (STEP == 2) asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (STEP == 2) copy(0, true, VB == 2);
+    if (KB == 2) copy(0, true, VB == 2);
 
     float* const pw = prow + (grp * kBr + wrow) * kBc;                      // this warp's weights
     float m[R], l[R], o[R][DPL];
@@ -133,7 +133,7 @@ fa_step_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __rest
 
     const int steps = (ntiles + G - 1) / G;
     for (int j = 0; j < steps; ++j) {
-        const int buf = STEP == 2 ? (j & 1) : 0, live = min(kBc, seq_k - (j * G + grp) * kBc);
+        const int buf = KB == 2 ? (j & 1) : 0, live = min(kBc, seq_k - (j * G + grp) * kBc);
         const unsigned char* Kc = Kt + (buf * G + grp) * Sh::K_BYTES;
         const unsigned char* Vc = Vt + (j % VB * G + grp) * Sh::V_BYTES;
         // no weight times whatever was there must be nothing
@@ -142,15 +142,19 @@ fa_step_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __rest
             uint4* Vl = reinterpret_cast<uint4*>(Vt + (j % VB * G + (ntiles - 1) % G) * Sh::V_BYTES);
             for (int i = seq_k % kBc * (Sh::ROW / 16) + threadIdx.x; i < kBc * (Sh::ROW / 16); i += kStepThreads) Vl[i] = make_uint4(0u, 0u, 0u, 0u);
         };
-        if (STEP == 2 && VB == 1) {                                        // V travels under the scores, the next K under the whole step
+        if (KB == 2 && VB == 1) {                                          // V travels under the scores, the next K under the whole step
             copy(j, false, true);
             if (j + 1 < steps) { copy(j + 1, true, false); asm volatile("cp.async.wait_group 2;" ::: "memory"); }
             else asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else if (STEP == 2) {                                            // prefetch the next tiles, wait for these
+        } else if (KB == 2) {                                              // prefetch the next tiles, wait for these
             if (j + 1 < steps) { copy(j + 1, true, true); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
             else asm volatile("cp.async.wait_group 0;" ::: "memory");
             clear_tail();
-        } else { copy(j, true, true); clear_tail(); }
+        } else {
+            copy(j, true, true);
+            if (STEP == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
+            clear_tail();
+        }
         __syncthreads();
         if (G == 1 || live > 0) {                                          // (the last step may have no tile for this group)
         // S[row][2l], S[row][2l+1]
@@ -195,7 +199,7 @@ fa_step_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __rest
         }
         __syncwarp();
         }
-        if (STEP == 2 && VB == 1) {
+        if (KB == 2 && VB == 1) {
             if (j + 1 < steps) asm volatile("cp.async.wait_group 1;" ::: "memory");
             else asm volatile("cp.async.wait_group 0;" ::: "memory");
             clear_tail();
@@ -388,12 +392,16 @@ int launch_step(const void* Q, const void* K, const void* V, void* O, int batch,
     const int G = seq_k > kBc ? Sh::MAX_G : 1;
     const unsigned grid = unsigned(batch) * heads * ((seq_q + kBr - 1) / kBr);
     // Step 2's fp32 tiles with one buffer of V leave room for a second CTA on an SM, if there is one (8 heads of 64, 512 keys: 36.0 us with two
-    // buffers, 28.3 with one; of 128: 68.9 and 58.9, but 1 head 35.0 and 36.8; fp16, 8 heads of 128: 47.2 and 50.1)
+    // buffers, 28.3 with one; of 128: 68.9 and 58.9, but 1 head 35.0 and 36.8; fp16, 8 heads of 128: 47.2 and 50.1).  Two groups' 16-bit tiles of
+    // 128 columns leave it with one buffer of either: the second CTA then computes while the first one copies.  fp16, 24 heads of 128, step 2 with one
+    // group, with two and two buffers, with two and one: 128 keys 15.3 / 16.5 / 13.5 us, 192 21.5 / 23.2 / 19.0, 512 142 / 137 / 117, 1024 505 / 473 / 408.
     constexpr int MOST = STEP == 2 ? 2 : 1;
-    const int VB = MOST == 2 && sizeof(T) == 4 && grid > unsigned(sm_count()) ? 1 : MOST;
-    const size_t smem = G * (size_t(MOST) * Sh::K_BYTES + size_t(VB) * Sh::V_BYTES) + (G * kBr * kBc + kBr * D) * sizeof(float);
-    auto kern = G == 2 ? fa_step_kernel<T, D, STEP, Sh::MAX_G, MOST> : fa_step_kernel<T, D, STEP, 1, MOST>;
-    if constexpr (sizeof(T) == 4) if (VB == 1) kern = G == 2 ? fa_step_kernel<T, D, STEP, Sh::MAX_G, 1> : fa_step_kernel<T, D, STEP, 1, 1>;
+    const bool share = STEP == 2 && grid > unsigned(sm_count()), one = share && sizeof(T) == 2 && G * D == 256;
+    const int KB = one ? 1 : MOST, VB = one || (share && sizeof(T) == 4) ? 1 : MOST;
+    const size_t smem = G * (size_t(KB) * Sh::K_BYTES + size_t(VB) * Sh::V_BYTES) + (G * kBr * kBc + kBr * D) * sizeof(float);
+    auto kern = G == 2 ? fa_step_kernel<T, D, STEP, Sh::MAX_G, MOST, MOST> : fa_step_kernel<T, D, STEP, 1, MOST, MOST>;
+    if constexpr (sizeof(T) == 4) if (VB < MOST) kern = G == 2 ? fa_step_kernel<T, D, STEP, Sh::MAX_G, MOST, 1> : fa_step_kernel<T, D, STEP, 1, MOST, 1>;
+    if constexpr (sizeof(T) == 2 && D == 128) if (KB < MOST) kern = fa_step_kernel<T, D, STEP, 2, 1, 1>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return int(e);

@@ -1,12 +1,13 @@
 """Step kernels whose warps are two groups that take every other tile of keys: one tile (one group), an odd number of tiles, a last tile of
-one key in either group's turn, scores that differ by much between the groups, and more CTAs than SMs (one buffer of V in step 2)."""
+one key in either group's turn, scores that differ by much between the groups, and more CTAs than SMs (step 2 has one buffer of V, in 16 bits and 128 columns one of K too)."""
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("S,heads", [(1, 1), (63, 3), (64, 2), (65, 1), (128, 1), (129, 5), (192, 1), (193, 40), (321, 2), (640, 8)])
+@pytest.mark.parametrize("S,heads", [(1, 1), (63, 3), (64, 2), (65, 1), (128, 1), (129, 5), (192, 1), (193, 40), (321, 2), (640, 8),
+                                     (128, 24), (192, 16), (256, 12), (320, 8), (384, 8)])                    # (128 ... 384: more CTAs than SMs)
 def test_groups(b200p, torch_cuda, S, heads, D):
     torch = torch_cuda
     g = torch.Generator(device="cuda").manual_seed(S + D)

@@ -5,6 +5,8 @@ import numpy as np
 import pytest
 
 from oracle import runtime_ref as rr
+import test_hybrid_gpu as hybrid
+from test_hybrid_gpu import knob, opened  # noqa: F401 (fixtures)
 from test_runtime_gpu import check_logits, to_device
 from test_skinny_sessions_gpu import llama
 
@@ -53,3 +55,17 @@ def test_rows_by_copies(b200p, torch_cuda, M, N, K):
     # products of 16-bit values are exact in fp32; K sums of them, each rounded: error below K eps of the sum of magnitudes, sqrt(K) of it in the mean
     bound = 2.0 ** -24 * 8 * K ** 0.5 * (X.double().abs() @ W.double().abs().T)
     assert ((out - want).abs() <= bound).all()
+
+
+# an MLP's rows that no kernel with the form takes: the sum comes from the GEMM, its folded form from a kernel of its own.  The first
+# layer's MLP is followed by a norm and the last one's by the head; 5 and 8 rows, 16 rows
+@pytest.mark.parametrize("batch", [5, 8, 16])
+def test_sums_of_the_gemm(b200p, torch_cuda, opened, knob, batch):  # noqa: F811
+    knob("skinny_cluster", 1)
+    s, cfg = opened("wide_mlp", "bf16", 64, batch), hybrid.CONFIGS["wide_mlp"]
+    ids = [hybrid.tokens(cfg, 9, b) for b in range(batch)]
+    got = [s.extend([i[:3] for i in ids], [2])]
+    for t in range(3, 9):
+        got.append(s.extend([i[t:t + 1] for i in ids], [0]))
+    for b in range(batch):
+        hybrid.check(np.concatenate([g[b] for g in got]), hybrid.reference("wide_mlp", ids[b])[2:], "bf16", b)

@@ -152,8 +152,7 @@ constexpr int kSkinnyXPad = 8;        // elements: X rows are 16 bytes longer th
 __device__ __forceinline__ void skinny_barrier() { asm volatile("bar.sync 1, %0;" :: "r"(kSkinnyThreads) : "memory"); }
 
 // X into shared memory as 16-bit rows of K + kSkinnyXPad elements, rows in [M, Mp) zero; ends with a barrier.
-// HELD: quads of a row that a lane holds between the sum of squares and the scaling (PRO_RMSNORM).
-template <typename T, int PRO, bool EMB = false, int HELD = 4>
+template <typename T, int PRO, bool EMB = false>
 __device__ __forceinline__ void skinny_prologue(const SkinnyArgs& a, T* xs, float* part_ss, int Mp, int warp, int lane) {
     const int K = a.K, xstride = K + kSkinnyXPad;
     // ---- prologue: X into shared memory as 16-bit, rows in [M, Mp) zero --------------------------------
@@ -186,8 +185,10 @@ __device__ __forceinline__ void skinny_prologue(const SkinnyArgs& a, T* xs, floa
         }
     } else if (PRO == PRO_RMSNORM) {
         // forward.hpp:34-56: y = x * rsqrt(mean(x^2) + eps) * w.  8 / Mp warps share a row; each keeps
-        // up to HELD quads per lane in registers between the sum of squares and the scaling.
-        constexpr int CACHE = HELD;
+        // up to 4 quads per lane in registers between the sum of squares and the scaling.  (12, all of a latent of 1536
+        // columns, cost the rotated queries 61 registers: latent decoder of eight layers, a step, width 1024 with 1 sequence
+        // 245 -> 250 us, width 4096 with 8 sequences 886 -> 899.)
+        constexpr int CACHE = 4;
         const int wpr = kSkinnyWarps / Mp;                      // warps per row
         const int m = warp / wpr, part = warp % wpr;
         const int quads = K / 4, qper = (quads + wpr - 1) / wpr;
@@ -207,7 +208,6 @@ __device__ __forceinline__ void skinny_prologue(const SkinnyArgs& a, T* xs, floa
         if (m < a.M) {
             #pragma unroll
             for (int it = 0; it < CACHE; ++it) {
-                if (it >= 4 && q0 + 32 * it >= q1) break;
                 const int q = q0 + lane + 32 * it;
                 if (q < q1) {
                     cx[it] = ldx(q);
@@ -248,7 +248,6 @@ __device__ __forceinline__ void skinny_prologue(const SkinnyArgs& a, T* xs, floa
         if (m < a.M) {
             #pragma unroll
             for (int it = 0; it < CACHE; ++it) {
-                if (it >= 4 && q0 + 32 * it >= q1) break;
                 const int q = q0 + lane + 32 * it;
                 if (q < q1) put(q, cx[it], cw[it]);
             }
@@ -727,12 +726,13 @@ constexpr int kSkinnySlab = 2048;                  // columns of W per stage
 constexpr int kSkinnyStreamThreads = kSkinnyThreads + 32;
 constexpr int kSkinnyXBars = 4;                    // barriers of the copies of X
 
-// PAIR: two CTAs share an SM, each with one group and one stage (launch_skinny_mh).  Nine warps put five on one of an SM's four parts, so
-// that they have 96 registers at most, and the bound asks for them: with 97 and more the second half of the grid waits for the first,
-// without a ring to fetch ahead.  Unbounded, the folded, gated, rotated and post-norm forms take 98 to 153 registers; what holds them at
-// 96 without spills is two blocks of loads in flight instead of four, half the partial sums (K <= 2048) and four quads of a row.  Eight layers, a step
-// in us, before those forms grew / unbounded / bounded: latent, width 2048, 1 / 2 / 4 sequences 344 / 365 / 334, 367 / 400 / 359, 419 / 439 / 392;
-// Llama, width 1024, MLP 2048, 1 sequence 139 / 152 / 131; hybrid the same, 2 sequences 168 / 182 / 152; Llama, width 4096, 2048 columns of O, 259 / 270 / 248.
+// PAIR: two CTAs share an SM, each with one group and one stage (launch_skinny_mh).  Nine warps put five on one of an SM's
+// four parts, so that they have 96 registers at most, and the bound asks for them: with 97 and more the second half of the
+// grid waits for the first, without a ring to fetch ahead.  Unbounded, the folded forms take 96 to 99 registers and the post-norm
+// ones 121; what holds them at 96 without spills is two blocks of loads in flight instead of four and half the partial sums
+// (K <= 2048).  Eight layers, a step in us, before registers grew past 96 / after / bounded: latent, width 2048, 1, 2 and 4 sequences
+// 344 / 365 / 334, 367 / 400 / 359, 419 / 439 / 392; Llama, width 1024, MLP 2048, 1 sequence 139 / 152 / 131; hybrid of
+// the same sizes, 2 sequences 168 / 182 / 152; Llama, width 4096, 2048 columns of O, 2 sequences 259 / 270 / 248.
 template <typename T, int PRO, int EPI, int MH, bool PAIR>
 __global__ void __launch_bounds__(kSkinnyStreamThreads, PAIR ? 2 : 1)
 skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status, int* sticky) {
@@ -815,8 +815,7 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
             __syncwarp();
             if constexpr (PRO == PRO_SCALED) fold_load(a, warp, lane, sums);
         } else {
-            // (queries from a latent of up to 1536 columns, eight rows: one trip to memory)
-            skinny_prologue<T, PRO, false, EPI == EPI_PAIRROT && !PAIR ? 12 : 4>(a, xs, part_ss, Mp, warp, lane);
+            skinny_prologue<T, PRO>(a, xs, part_ss, Mp, warp, lane);
         }
         const int rows = pro_rows16(PRO) ? a.M : Mp;              // rows of X in shared memory
         const T* xrow = xs + size_t(g) * xstride + t4 * 16;

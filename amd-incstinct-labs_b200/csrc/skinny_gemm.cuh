@@ -758,15 +758,27 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
     const int ngroups = (epi_gated(EPI)) ? (a.N + 7) / 8 : (a.N + 15) / 16;
 
     // A CTA often starts when the last CTA of the kernel before leaves its SM, and what precedes the dependency wait is then part of
-    // the chain: the producer sets up the barriers and streams, the others go to the wait at once and meet it (barrier 2) afterwards.
+    // the chain.  Where X comes by copies the producer sets up the barriers and streams, and the others meet it (barrier 2) when they
+    // are about to ask for X.  Where it comes through registers all set out together: the first form is slower there (8 layers, a
+    // step in us, latent of width 1024 with 3 sequences 264 against 250, of 2048 with 1 and 4 333 / 391 against 319 / 369; projections of
+    // fp32 rows alone, 3 x 2560 x 2048 gated 9.7 against 8.4, 5 x 2048 x 2048 9.6 against 8.4), as the second is for copies (Llama of
+    // width 1024, 1 sequence, 147 against 143; hybrid of 1024, 1 sequence, 172 against 162).
+    constexpr bool copied = pro_rows16(PRO);
+    auto set_up = [&] {
+        for (int s = 0; s < nstages; ++s) { dme::mbar_init(&full_bar[s], 1); dme::mbar_init(&empty_bar[s], kSkinnyWarps); }
+        if (copied) for (int s = 0; s < kSkinnyXBars; ++s) dme::mbar_init(&x_bar[s], 1);
+        dme::mbar_init_fence();
+    };
+    if constexpr (!copied) {
+        if (threadIdx.x == 0) set_up();
+        __syncthreads();
+    }
     if (warp == kSkinnyWarps) {
-        if (lane == 0) {
-            for (int s = 0; s < nstages; ++s) { dme::mbar_init(&full_bar[s], 1); dme::mbar_init(&empty_bar[s], kSkinnyWarps); }
-            for (int s = 0; s < kSkinnyXBars; ++s) dme::mbar_init(&x_bar[s], 1);
-            dme::mbar_init_fence();
+        if constexpr (copied) {
+            if (lane == 0) set_up();
+            __syncwarp();
+            asm volatile("bar.arrive 2, %0;" :: "n"(kSkinnyStreamThreads) : "memory");
         }
-        __syncwarp();
-        asm volatile("bar.arrive 2, %0;" :: "n"(kSkinnyStreamThreads) : "memory");
         // ---- producer: W is constant, so it streams before and through the dependency wait of the consumers ----
         if (lane == 0) {
             const uint64_t pol = dme::policy_evict_first();
@@ -798,7 +810,7 @@ skinny_stream_kernel(const SkinnyArgs a, int nstages, int slab_cols, int* status
         EpiAhead<MH> ahead;
         float4 sums[PRO == PRO_SCALED ? MH : 1][PAIR ? 2 : 4];
         if (EPI != EPI_ROPE) skinny_epilogue_fetch_constants<T, EPI, MH>(a, blockIdx.x, threadIdx.x, ahead);
-        asm volatile("bar.sync 2, %0;" :: "n"(kSkinnyStreamThreads) : "memory");       // the mbarriers are there
+        if constexpr (copied) asm volatile("bar.sync 2, %0;" :: "n"(kSkinnyStreamThreads) : "memory");       // the mbarriers are there
         // 16-bit rows of X: one bulk copy per row and slab (a barrier each for the first slabs, the last for the rest).  Through
         // registers they came in batches, one trip to L2 after the other (16 rows of 2048: eight, 3.4 us; 1.3 by copies)
         if (pro_rows16(PRO) && threadIdx.x == 0)

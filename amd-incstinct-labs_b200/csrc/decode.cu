@@ -22,8 +22,9 @@
 //  * the online softmax runs per warp and per tile: one running max per head
 //    shared by the warp (wave::dpp::reduce_max style butterfly over the lane
 //    groups), O rescaled at most once per tile and only when a max moved;
-//  * warps are merged through shared memory, splits through a workspace and a
-//    small combine kernel, both with the reference's merge
+//  * warps are merged through shared memory; splits of a unit (sequence, KV head) as one thread-block cluster through
+//    distributed shared memory (513 .. 2048 keys), through a workspace by the last CTA of the unit, or, for fp32 partials and for
+//    other ranks, by a small combine kernel; all with the reference's merge
 //    m = max m_w; l = sum e^{m_w-m} l_w; O = sum e^{m_w-m} O_w / l
 //    (fa_decode_kernel.hpp:75-92).
 // HBM-bound: algorithmic bytes = K and V once + q + o.
@@ -856,7 +857,9 @@ DecodePlan plan_decode(int D, int N, int nQH, int nKVH, int batch, bool clusters
         // For 513 to 2048 keys the splits of a unit are one cluster, as large as lets all units run at a time.  Calls replayed from
         // a graph, cold keys, without and with, 32 / 8 heads of 128: 1 sequence, 700 / 1000 / 2048 keys 9.3 / 10.3 / 10.3 -> 8.3 / 8.3 / 8.4 us;
         // 4 sequences 10.1 / 10.7 / 17.3 -> 8.4 / 10.0 / 13.1; 8 sequences, two CTAs a cluster, 10.3 / 12.3 / 26.7 -> 11.1 / 12.4 / 16.7, so
-        // pairs only above 1024; under 512 a cluster costs more than one CTA's tiles (256 keys: 6.6 -> 7.9).
+        // pairs only above 1024; under 512 a cluster costs more than one CTA's tiles (256 keys: 6.6 -> 7.9).  The upper end is not where
+        // the other form wins (2304 / 4096 keys, 1 sequence 10.4 / 10.3 against 9.2 / 10.2 us, 4 sequences 16.5 / 24.8 against 10.3 /
+        // 16.5) but how far this one has been compared in 64 bits: a cluster's splits grow with the keys, the others stay at 256 or so.
         if (clusters && N > 512 && N <= 2048) {
             int c = (N + 127) / 128 < kMaxCluster ? (N + 127) / 128 : kMaxCluster;
             while (c > 1 && stc_resident_clusters(c) < units) --c;

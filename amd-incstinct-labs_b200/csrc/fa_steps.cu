@@ -50,14 +50,14 @@ template <> __device__ __forceinline__ float exp_for<__half>(float x)        { r
 template <> __device__ __forceinline__ float exp_for<__nv_bfloat16>(float x) { return __expf(x); }
 
 // What bounds this kernel is shared memory: a warp reads the whole K and V tile for its rows, and q and the weights as broadcasts.
-// Four rows of a warp share each read (12 wavefronts for 32 FMAs; two rows 20, one row 40 KB per row and tile), and so that
-// there are still eight warps for 16 rows, they are two groups that take every other tile; the second group's maxima, sums and O join
-// the first's at the end.  (fp32 heads of 128: one group of two rows a warp, two tiles would
-// leave no second CTA.)  Every lane reads
-// its own two key rows at the same 16-byte chunk, so q is a broadcast; the keys lie 16 bytes further apart than their size, odd keys
-// behind the even ones, and the eight lanes of a shared-memory phase hit eight different bank groups.  Against one group of two
-// rows a warp, graph replays, step 1 / step 2: 8 heads of 64, 512 keys, fp32 37.9 / 34.5 -> 29.4 / 28.2 us, fp16 30.4 / 30.0 -> 26.7 / 25.0;
-// 24 heads, 1024 keys, fp32 352 / 327 -> 300 / 279; fp16, heads of 128, 498 / 505 -> 438 / 479.
+// Two 16-byte reads of K per lane (8 wavefronts) serve all rows of the warp, each row's q one more: 32 FMAs a lane cost 12 wavefronts
+// with four rows, 20 with two and 36 with one.  So that there are still eight warps for 16 rows, they are two groups
+// that take every other tile; the second group's maxima, sums and O join the first's at the end.  (fp32 heads of 128: one group of two
+// rows a warp, two tiles would leave no second CTA.)  Every lane reads its own two key rows at the same 16-byte chunk, so q is a
+// broadcast; the keys lie 16 bytes further apart than their size, odd keys behind the even ones, and the eight lanes of a
+// shared-memory phase hit eight different bank groups.  Against one group of two rows a warp, graph replays, step 1 / step 2: 8 heads of
+// 64, 512 keys, fp32 37.9 / 34.3 -> 30.6 / 29.1 us, fp16 30.7 / 30.5 -> 25.7 / 24.6; 24 heads, 1024 keys, fp32 353 / 327 -> 306 / 287;
+// fp16, heads of 128, 497 / 505 -> 431 / 408.  Counted for the first of these, fp32, step 2: 6.6 -> 4.6 million wavefronts.
 // Lengths need not be multiples of the tiles: keys past the end get no weight, rows past the end are not stored.
 constexpr int kStepWarps = 8, kStepThreads = kStepWarps * 32;
 template <typename T, int D> struct StepTile {
@@ -68,8 +68,11 @@ template <typename T, int D> struct StepTile {
 };
 
 // G groups of warps, KB and VB buffers of their tiles of K and V (step 2: 2 and 2, 2 and 1, or 1 and 1; the others: 1 and 1)
+// CTAs an SM the registers are bound for: fp32 heads of 128, steps 1 and 2, 8 heads, 512 keys, 64.7 and 60.6 us with 2, 62.8 and 58.9 with
+// 1.  (Unbound, with 60 registers, they take 2 to 3 % less where all rounds of CTAs are full, and up to a quarter more where the last one
+// is not: 8 heads, 512 / 831 keys, step 1 63.0 / 195 against 64.7 / 160 us.)
 template <typename T, int D, int STEP, int G, int KB, int VB>
-__global__ void __launch_bounds__(kStepThreads, D * sizeof(T) > 256 && STEP != 0 ? 1 : 2)      // (fp32 heads of 128, steps 1 and 2, 8 heads, 512 keys: 64.7 and 60.6 us with 2, 62.8 and 58.9 with 1)
+__global__ void __launch_bounds__(kStepThreads, D * sizeof(T) > 256 && STEP != 0 ? 1 : 2)
 fa_step_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V, T* __restrict__ O,
                int seq_q, int seq_k, int heads, float scale, float m_first) {
     using Sh = StepTile<T, D>;

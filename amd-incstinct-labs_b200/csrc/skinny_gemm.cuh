@@ -109,8 +109,10 @@ struct SkinnyPairRot {
 // projection is W . (x * inv * w) = inv * (W . (x * w)) with one inv per row, so whoever adds to x (EPI_ADD_FOLD: each CTA
 // its columns) rounds x * w once for all readers, and a reader copies 16-bit rows and scales its sums.  As a prologue
 // (PRO_RMSNORM) every CTA reads all of x in fp32 and, from eight rows on, goes through it twice.  Decode step of 22 layers of width
-// 2048, 2 / 8 / 16 sequences: 0.576 / 0.737 / 0.998 ms with the prologues, 0.560 / 0.597 / 0.803 folded; 8 layers of width 4096, 2 sequences: 0.685, 0.644.  The rounding is the same size: one 16-bit rounding per operand, whose exponent does not matter to
-// bf16; fp16 could overflow ahead of the scale, so fp16 sessions keep the prologue.
+// 2048, 2 / 8 / 16 sequences: 0.576 / 0.737 / 0.998 ms with the prologues, 0.560 / 0.597 / 0.803 folded; 8 layers of width
+// 4096, 2 sequences: 0.685, 0.644.  The rounding is the same size: one 16-bit rounding per operand, whose exponent does not matter
+// to bf16 (against 64 bits, 12 seeds each, before and folded: Llama of width 2048 0.00557 and 0.00556, hybrid of 1024 0.00467 and
+// 0.00456); fp16 could overflow ahead of the scale, so fp16 sessions keep the prologue.
 struct SkinnyFold {
     const float* ss;       // PRO_SCALED: [M][ss_ld] sums of squares of a row over disjoint columns, `parts` of them
     int parts, ss_ld;

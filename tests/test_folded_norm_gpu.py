@@ -1,6 +1,7 @@
 """Decode steps whose norms are folded into the projections around them (bf16): x * w rounded by whoever adds to x, 1 / rms from
 partial sums.  Sizes where the partial sums end inside a vector, pass the vectors a lane loads at once or are made by the kernel that
-splits K; one and two fragments of rows; and rows of X by bulk copies, with half stages where X leaves room for one whole stage only."""
+splits K; one and two fragments of rows; sums that only the GEMM takes; and rows of X by bulk copies, with half stages where X leaves room
+for one whole stage only."""
 import numpy as np
 import pytest
 
